@@ -57,13 +57,13 @@ def listed():
         dict(name="loss-1297x840", kind="loss", width=1297, height=840, u8=True),
         # Training the small multi-view scene once it has grown: 256x256 views.
         dict(name="train-blobs", kind="train", scene="blobs", n=34380, width=256, height=256, views=16, batch=1,
-             iterations=10, bf16=False, fp64_conic=False),
+             iterations=30, bf16=False, fp64_conic=False),
         # Training the clustered scene at 1297x840 at its converged size.
         dict(name="train-shells", kind="train", scene="shells", n=187001, width=1297, height=840, views=6, batch=1,
-             iterations=5, bf16=False, fp64_conic=False),
+             iterations=20, bf16=False, fp64_conic=False),
         # Batched mixed-size training: 8 views a step, BF16 storage, f64 conics.
         dict(name="train-batch", kind="train", scene="shells", n=100000, width=0, height=0, views=12, batch=8,
-             iterations=2, bf16=True, fp64_conic=True),
+             iterations=4, bf16=True, fp64_conic=True),
         # Learned densification at an event: all Gaussians scored, one gradient of 65,536 records.
         dict(name="policy-500k", kind="policy", n=500000, records=65536),
     ]
@@ -87,9 +87,9 @@ def draw(rng):
         width, height = max(128, width * 2 // 3), max(96, height * 2 // 3)
         if rng.random() < 0.3:
             return dict(kind=kind, scene=scene, n=_log_int(rng, 2000, 100000 if scene != "blobs" else 35000), width=0,
-                        height=0, views=9, batch=rng.randint(2, 8), iterations=2, bf16=True, fp64_conic=True)
+                        height=0, views=9, batch=rng.randint(2, 8), iterations=4, bf16=True, fp64_conic=True)
         return dict(kind=kind, scene=scene, n=_log_int(rng, 2000, 187000 if scene != "blobs" else 35000), width=width,
-                    height=height, views=rng.randint(3, 12), batch=1, iterations=rng.randint(4, 8),
+                    height=height, views=rng.randint(3, 12), batch=1, iterations=rng.randint(10, 20),
                     bf16=rng.random() < 0.25, fp64_conic=rng.random() < 0.25)
     most = {"blobs": 35000, "box": 1000000, "shells": 500000}[scene]
     if kind == "host":
