@@ -88,80 +88,77 @@ CRM_HD float expf_cr(float x) {
   return (float)(p * s);
 }
 
-// 2^(j/64), j = 0..63, each correctly rounded to double.
-#define CRM_EXP2_TAB64                                                                          \
-  {0x1.0000000000000p+0, 0x1.02c9a3e778061p+0, 0x1.059b0d3158574p+0, 0x1.0874518759bc8p+0,     \
-   0x1.0b5586cf9890fp+0, 0x1.0e3ec32d3d1a2p+0, 0x1.11301d0125b51p+0, 0x1.1429aaea92de0p+0,     \
-   0x1.172b83c7d517bp+0, 0x1.1a35beb6fcb75p+0, 0x1.1d4873168b9aap+0, 0x1.2063b88628cd6p+0,     \
-   0x1.2387a6e756238p+0, 0x1.26b4565e27cddp+0, 0x1.29e9df51fdee1p+0, 0x1.2d285a6e4030bp+0,     \
-   0x1.306fe0a31b715p+0, 0x1.33c08b26416ffp+0, 0x1.371a7373aa9cbp+0, 0x1.3a7db34e59ff7p+0,     \
-   0x1.3dea64c123422p+0, 0x1.4160a21f72e2ap+0, 0x1.44e086061892dp+0, 0x1.486a2b5c13cd0p+0,     \
-   0x1.4bfdad5362a27p+0, 0x1.4f9b2769d2ca7p+0, 0x1.5342b569d4f82p+0, 0x1.56f4736b527dap+0,     \
-   0x1.5ab07dd485429p+0, 0x1.5e76f15ad2148p+0, 0x1.6247eb03a5585p+0, 0x1.6623882552225p+0,     \
-   0x1.6a09e667f3bcdp+0, 0x1.6dfb23c651a2fp+0, 0x1.71f75e8ec5f74p+0, 0x1.75feb564267c9p+0,     \
-   0x1.7a11473eb0187p+0, 0x1.7e2f336cf4e62p+0, 0x1.82589994cce13p+0, 0x1.868d99b4492edp+0,     \
-   0x1.8ace5422aa0dbp+0, 0x1.8f1ae99157736p+0, 0x1.93737b0cdc5e5p+0, 0x1.97d829fde4e50p+0,     \
-   0x1.9c49182a3f090p+0, 0x1.a0c667b5de565p+0, 0x1.a5503b23e255dp+0, 0x1.a9e6b5579fdbfp+0,     \
-   0x1.ae89f995ad3adp+0, 0x1.b33a2b84f15fbp+0, 0x1.b7f76f2fb5e47p+0, 0x1.bcc1e904bc1d2p+0,     \
-   0x1.c199bdd85529cp+0, 0x1.c67f12e57d14bp+0, 0x1.cb720dcef9069p+0, 0x1.d072d4a07897cp+0,     \
-   0x1.d5818dcfba487p+0, 0x1.da9e603db3285p+0, 0x1.dfc97337b9b5fp+0, 0x1.e502ee78b3ff6p+0,     \
-   0x1.ea4afa2a490dap+0, 0x1.efa1bee615a27p+0, 0x1.f50765b6e4540p+0, 0x1.fa7c1819e90d8p+0}
+// Correctly rounded e^-s for the compositing range 0 <= s <= kExpGridMax, for hot loops:
+// s = n/128 + t with n = rint(128 s), so |t| <= 2^-8 and t is exact in float (a multiple of
+// ulp(s) no larger than s); e^-s = E[n] (1 + q), E[n] = e^(-n/128) rounded to double, q =
+// e^-t - 1 by its Taylor series to t^5 (truncation below 5e-18 relative). The only double
+// operations are the six of the series and the two conversions; the reduction is three
+// float operations. An exhaustive sweep over every float in [0, kExpGridMax] gives results
+// identical to expf_cr. `tab` holds kExpGridEntries values; the last one is 0, so that s =
+// kExpGridSkip gives exactly 0.
+constexpr float kExpGridMax = 6.2f;  // ln(255) = 5.54 is the largest argument of opacity <= 1
+constexpr int kExpGridEntries = 796;  // n = 0..rint(6.2 * 128), then the zero
+constexpr float kExpGridSkip = 6.2109375f;    // 795 / 128
+constexpr float kExpGridMagic = 12582912.0f;  // 1.5 * 2^23: adding it rounds to an integer
 
-// The same correctly rounded e^x with fewer double operations, for hot loops (table-driven
-// method, Tang 1989): x = (64 m + j) ln2/64 + r with |r| <= ln2/128, ln2/64 split into a
-// 39-bit head and a tail (so the head product and x minus it are exact);
-// e^x = 2^m * 2^(j/64) * (1 + q), q = e^r - 1 by its Taylor series to r^5 (truncation
-// below 4e-17 relative). `tab` is CRM_EXP2_TAB64 (in shared memory on the device). An
-// exhaustive sweep over every float in [-110, 90] gives results identical to expf_cr.
-CRM_HD float expf_cr_tab(float x, const double* tab) {
-  if (!(x == x)) return x;
-  if (x > 88.8f) return (float)INFINITY;
-  if (x < -104.0f) return 0.0f;
-  double d = (double)x;
-  double n = rint(d * 0x1.71547652b82fep+6);  // 64 / ln2
-  double r = fma(-n, 0x1.62e42fefa0000p-7, d);
-  r = fma(-n, 0x1.cf79abc9e3b3ap-46, r);
-  int ni = (int)n;
-  double c = fma(r, 0x1.1111111111111p-7, 0x1.5555555555555p-5);  // 1/120, 1/24
-  c = fma(r, c, 0x1.5555555555555p-3);                            // 1/6
-  c = fma(r, c, 0.5);
-  c = fma(r, c, 1.0);
-  double q = r * c;
-  double t = tab[ni & 63];
-  double y = fma(t, q, t);
-  double s = bits_to_double((uint64_t)((ni >> 6) + 1023) << 52);
-  return (float)(y * s);
+// The series: e^-t - 1 for |t| <= 2^-8, times E.
+CRM_HD float exp_grid_finish(float t, double e) {
+  const double d = (double)t;
+  double c = fma(d, -0x1.1111111111111p-7, 0x1.5555555555555p-5);  // -1/120, 1/24
+  c = fma(d, c, -0x1.5555555555555p-3);                            // -1/6
+  c = fma(d, c, 0.5);
+  c = fma(d, c, -1.0);
+  const double q = d * c;
+  return (float)fma(e, q, e);
 }
 
-// expf_cr_tab for the compositing range. The argument there is -sigma with
-// 0 <= sigma <= sigma_max = ln(255 * opacity) <= ln 255, so n = rint(64 x / ln2) lies in
-// [-512, 0]. A table of 2^(n/64) for n in [-(kExpNegEntries-1), 0] folds the 2^m scale into
-// the table entry (entry k = table64[(-k) & 63] * 2^((-k) >> 6), exact), so
-// fma(t', q, t') = 2^m * fma(t, q, t) exactly and the result equals expf_cr_tab bit for
-// bit; arguments below kExpNegMin (never produced by a valid projection) and NaN take
-// expf_cr.
-constexpr int kExpNegEntries = 577;
-constexpr float kExpNegMin = -6.2f;  // rint(-6.2 * 64 / ln2) = -572
-
-CRM_HD double exp2_neg_entry(int k, const double* tab64) {
-  const int n = -k;
-  return bits_to_double(double_to_bits(tab64[n & 63]) + ((uint64_t)(int64_t)(n >> 6) << 52));
+CRM_HD float expf_cr_grid(float s, const double* tab) {
+  const float m = fmaf(s, 128.0f, kExpGridMagic);
+  const float nf = m - kExpGridMagic;
+  const float t = fmaf(nf, -0.0078125f, s);  // exact
+  return exp_grid_finish(t, tab[(int)nf]);
 }
 
-CRM_HD float expf_cr_neg(float x, const double* tab_neg) {
-  if (!(x >= kExpNegMin)) return expf_cr(x);
-  const double d = (double)x;
-  const double n = rint(d * 0x1.71547652b82fep+6);  // 64 / ln2
-  double r = fma(-n, 0x1.62e42fefa0000p-7, d);
-  r = fma(-n, 0x1.cf79abc9e3b3ap-46, r);
-  double c = fma(r, 0x1.1111111111111p-7, 0x1.5555555555555p-5);  // 1/120, 1/24
-  c = fma(r, c, 0x1.5555555555555p-3);                            // 1/6
-  c = fma(r, c, 0.5);
-  c = fma(r, c, 1.0);
-  const double q = r * c;
-  const double t = tab_neg[-(int)n];
-  return (float)fma(t, q, t);
-}
+// E[n], built at compile time in double-double arithmetic (error-free sums and products,
+// Dekker 1971): e^(-1/128) by its Taylor series, then its powers.
+struct ExpGrid {
+  double v[kExpGridEntries];
+  struct dd {
+    double h, l;
+  };
+  static constexpr dd fast_two_sum(double a, double b) {
+    const double s = a + b;
+    return dd{s, b - (s - a)};
+  }
+  static constexpr dd two_prod(double a, double b) {
+    const double ca = 134217729.0 * a, cb = 134217729.0 * b;
+    const double ah = ca - (ca - a), al = a - ah, bh = cb - (cb - b), bl = b - bh;
+    const double p = a * b;
+    return dd{p, ((ah * bh - p) + ah * bl + al * bh) + al * bl};
+  }
+  static constexpr dd mul(dd a, dd b) {
+    const dd p = two_prod(a.h, b.h);
+    return fast_two_sum(p.h, p.l + (a.h * b.l + a.l * b.h));
+  }
+  static constexpr dd div_int(dd a, double k) {  // a / k for a small integer k
+    const double q = a.h / k;
+    const dd p = two_prod(q, k);
+    return fast_two_sum(q, (((a.h - p.h) - p.l) + a.l) / k);
+  }
+  constexpr ExpGrid() : v() {
+    dd term{1.0, 0.0}, sum{1.0, 0.0};
+    for (int k = 1; k <= 14; k++) {
+      term = div_int(dd{term.h * -0.0078125, term.l * -0.0078125}, (double)k);
+      const dd s = fast_two_sum(sum.h, term.h);
+      sum = fast_two_sum(s.h, s.l + sum.l + term.l);
+    }
+    dd p{1.0, 0.0};
+    for (int n = 0; n < kExpGridEntries; n++) {
+      v[n] = n < kExpGridEntries - 1 ? p.h : 0.0;
+      p = mul(p, sum);
+    }
+  }
+};
 
 // Correctly rounded natural log for float x.
 CRM_HD float logf_cr(float x) {

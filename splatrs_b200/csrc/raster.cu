@@ -1,15 +1,20 @@
 // Front-to-back alpha compositing, forward and backward (reference src/rasterize.rs).
 //
-// One block per tile (16x16 by default; 8x8 and 16x32 too), one pixel per thread. Warps own
-// 8x4 pixel sub-blocks so that an entry whose pixel rectangle misses a sub-block is skipped
-// by the whole warp with one uniform branch. The tile's sorted entries are staged through
-// shared memory in chunks of CH entries (32-256; each entry's 48-byte record gathered by one
-// thread). Tile shape and chunk depth are template parameters, chosen at run time from the
-// context's configuration (the autotuner's pick). Every
-// per-pixel decision (sigma range, alpha >= 1/255, the 0.99 clamp, T < 1e-4) is taken on
-// values computed exactly as the reference computes them: unfused arithmetic and a
-// correctly rounded exp.
+// The forward and the default backward give every warp an 8x8 pixel sub-block of a tile (two
+// pixels per lane, computed as f32x2 pairs) and let it walk the tile's sorted list by itself:
+// it scans 64 entries at a time for those whose pixel rectangle touches its sub-block, stages
+// their records 32 at a time in its own shared memory (gathered while the previous 32 are
+// composited) and never meets the block's other warps at a barrier. The one-pixel-per-thread
+// backward and the deterministic one run one block per tile instead and stage chunks for the
+// whole block. Tile shape (16x16 by default; 8x8 and 16x32 too) and, for the one-pixel
+// backward, chunk depth are template parameters chosen at run time from the context's
+// configuration (the autotuner's pick). Every per-pixel decision (sigma range, alpha >= 1/255,
+// the 0.99 clamp, T < 1e-4) is taken on values computed exactly as the reference computes
+// them: unfused arithmetic and a correctly rounded exp.
+#include <mutex>
+#include <set>
 #include <type_traits>
+#include <utility>
 
 #include "common.cuh"
 #include "kernels.cuh"
@@ -31,48 +36,8 @@ struct TileGeo {
   static_assert(TW % 8 == 0 && TH % 4 == 0 && TW <= 16 && TH <= 32, "tile shape");
 };
 
-struct PixelGeom {
-  uint32_t px_i, py_j;   // absolute pixel
-  uint32_t bx0, by0;     // warp sub-block origin
-  bool inside;
-};
-
-template <int TW, int TH>
-__device__ __forceinline__ PixelGeom pixel_geom(uint32_t tile, uint32_t tiles_x, uint32_t width, uint32_t height) {
-  constexpr int WX = TileGeo<TW, TH>::kWarpsX;
-  const uint32_t tx = tile % tiles_x, ty = tile / tiles_x;
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  PixelGeom p;
-  p.bx0 = tx * TW + (warp % WX) * 8u;
-  p.by0 = ty * TH + (warp / WX) * 4u;
-  p.px_i = p.bx0 + (lane & 7u);
-  p.py_j = p.by0 + (lane >> 3);
-  p.inside = p.px_i < width && p.py_j < height;
-  return p;
-}
-
-
-__constant__ double kExp2Tab64[64] = CRM_EXP2_TAB64;
-
-// evaluate (rasterize.rs:231-244). Returns false when skipped. `tab` is the table of
-// crm::expf_cr_neg in shared memory.
-__device__ __forceinline__ bool evaluate(float px, float py, float mx, float my, float A, float B, float C,
-                                         float opacity, float sigma_max, const double* tab, float* gauss_out,
-                                         float* alpha_out) {
-  const float dx = px - mx;
-  const float dy = py - my;
-  const float sigma = 0.5f * (A * dx * dx + C * dy * dy) + B * dx * dy;
-  if (sigma < 0.0f || sigma > sigma_max) return false;
-  const float gauss = crm::expf_cr_neg(-sigma, tab);
-  const float og = opacity * gauss;
-  if (og < SPLAT_ALPHA_MIN) return false;
-  *gauss_out = gauss;
-  *alpha_out = fminf(og, SPLAT_ALPHA_MAX);
-  return true;
-}
-
-// evaluate (rasterize.rs:231-244) with the general correctly rounded exp: same values and
-// decisions as evaluate() (the narrow-range table form equals it on the whole argument range).
+// evaluate (rasterize.rs:231-244), scalar, with the general correctly rounded exp. Returns
+// false when skipped.
 __device__ __forceinline__ bool evaluate_ref(float px, float py, float mx, float my, float A, float B, float C,
                                              float opacity, float sigma_max, float* gauss_out, float* alpha_out) {
   const float dx = px - mx;
@@ -268,21 +233,6 @@ __device__ __forceinline__ uint32_t subblock_mask(uint32_t rx, uint32_t ry, uint
   return m;
 }
 
-// 32x32 bit-matrix transpose across a warp: lane j holds row j on entry; on return lane L
-// holds column L (bit j of the result = bit L of lane j's input). Five exchange stages,
-// each swapping the off-diagonal blocks of size s.
-__device__ __forceinline__ uint32_t warp_transpose_bits(uint32_t x) {
-  const uint32_t lane = threadIdx.x & 31;
-  const uint32_t masks[5] = {0x0000ffffu, 0x00ff00ffu, 0x0f0f0f0fu, 0x33333333u, 0x55555555u};
-#pragma unroll
-  for (int i = 0; i < 5; i++) {
-    const uint32_t sh = 16u >> i, m = masks[i];
-    const uint32_t y = __shfl_xor_sync(0xffffffffu, x, sh);
-    x = (lane & sh) ? ((x & ~m) | ((y & ~m) >> sh)) : ((x & m) | ((y & m) << sh));
-  }
-  return x;
-}
-
 // Compacts, in order, the chunk-local indices k < cnt whose mask has this warp's bit (and,
 // when `limit` is finite, k < limit) into list[]; returns how many.
 template <typename WM>
@@ -302,115 +252,362 @@ __device__ __forceinline__ uint32_t build_warp_list(const WM* __restrict__ smask
   return n;
 }
 
-// forward_tile (rasterize.rs:249-302) for one tile per block. Each warp walks, 32 at a
-// time, the chunk's entries whose pixel rectangle touches its 8x4 sub-block; a lane takes
-// only the entries whose rectangle covers its own pixel (the rectangle test of the
-// reference), found from the batch's coverage masks transposed across the warp, so the
-// warp runs as many rounds as its busiest lane rather than one round per entry. Each lane
-// still composites its entries in list (depth) order. kCount adds the evaluated-pair counter
-// (untimed diagnostics only).
-template <int TW, int TH, int CH, bool kCount>
-__global__ void __launch_bounds__(TW * TH, 1536 / (TW * TH)) raster_fwd_kernel(
-    const float4* __restrict__ rec, const uint32_t* __restrict__ gauss, const uint2* __restrict__ ranges,
-    uint32_t width, uint32_t height, uint32_t tiles_x, float bg0, float bg1, float bg2, float* __restrict__ image,
-    float* __restrict__ final_t, uint32_t* __restrict__ n_contrib, unsigned long long* __restrict__ pairs,
-    const BatchTable* __restrict__ bt) {
-  typedef TileGeo<TW, TH> Geo;
-  constexpr int NT = Geo::kThreads;
-  if (bt && blockIdx.x >= bt->tile_start[bt->views]) return;  // past the batch's tiles
-  __shared__ float4 s0[CH], s1[CH];
-  __shared__ float2 s2[CH];
-  __shared__ typename Geo::Mask srect[CH];
-  __shared__ typename Geo::WarpMask smask[CH];
-  __shared__ uint8_t slist[Geo::kWarps][CH];
-  __shared__ double stab[crm::kExpNegEntries];
-  for (int i = threadIdx.x; i < crm::kExpNegEntries; i += NT) stab[i] = crm::exp2_neg_entry(i, kExp2Tab64);
-  // In a batch the block is a global tile: find its view, local tile and image offset.
-  uint32_t tile = blockIdx.x;
-  size_t pix0 = 0;
-  if (bt) {
-    const int v = batch_view_of(bt->tile_start, bt->views, blockIdx.x);
-    tile = blockIdx.x - bt->tile_start[v];
-    width = bt->cam[v].width;
-    height = bt->cam[v].height;
-    tiles_x = bt->tiles_x[v];
-    pix0 = bt->pix_start[v];
-  }
-  const PixelGeom pg = pixel_geom<TW, TH>(tile, tiles_x, width, height);
-  const uint32_t ox = (tile % tiles_x) * TW, oy = (tile / tiles_x) * TH;
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // Sub-block origin in the tile; its rows' bits in the rectangle masks.
-  const uint32_t sbx = (warp % Geo::kWarpsX) * 8u, sby = (warp / Geo::kWarpsX) * 4u + Geo::kRowShift;
-  const float px = (float)pg.px_i + 0.5f, py = (float)pg.py_j + 0.5f;
-  const uint2 range = ranges[blockIdx.x];
-  uint8_t* list = slist[warp];
-  float T = 1.0f, cr = 0.0f, cg = 0.0f, cb = 0.0f;
-  uint32_t ncon = 0;
-  bool done = !pg.inside;
-  unsigned long long npairs = 0;
-  for (uint32_t base = range.x; base < range.y; base += CH) {
-    if (__syncthreads_count(!done) == 0) break;
-#pragma unroll
-    for (uint32_t e = threadIdx.x; e < (uint32_t)CH; e += NT) {
-      const uint32_t idx = base + e;
-      uint32_t m = 0;
-      if (idx < range.y) {
-        const uint32_t g = gauss[idx];
-        s0[e] = rec[4 * (size_t)g];
-        s1[e] = rec[4 * (size_t)g + 1];
-        const float4 e2 = rec[4 * (size_t)g + 2];
-        s2[e] = make_float2(e2.x, e2.y);
-        srect[e] = tile_rect_masks<TW, TH>(fbits(e2.z), fbits(e2.w), ox, oy);
-        m = subblock_mask<TW, TH>(fbits(e2.z), fbits(e2.w), ox, oy);
-      }
-      smask[e] = (typename Geo::WarpMask)m;
+// ---------------------------------------------------------------------------------------
+// A tile's list and the warps' walk of it, shared by the forward and the paired backward.
+// ---------------------------------------------------------------------------------------
+constexpr int kListChunk = 1024;  // list entries scanned at once: most tiles take one scan
+constexpr int kStage = 32;        // entries staged per round, one per lane
+constexpr int kQueue = 64;        // hits waiting to be staged: up to 31 + one step of 32
+
+// Part of a tile's list in shared memory: every entry's Gaussian and the sub-blocks of the
+// tile its pixel rectangle touches (one bit each).
+template <typename Mask>
+struct TileList {
+  uint32_t g[kListChunk];
+  Mask mask[kListChunk];
+};
+
+// Geometry of one warp's 8 x BH pixel sub-block: kPerTile warps share a tile.
+template <int TW, int TH, int BH>
+struct Walk {
+  static constexpr int kPerTile = TW * TH / (8 * BH), kAcross = TW / 8;
+  typedef typename std::conditional<(kPerTile > 8), uint16_t, uint8_t>::type Mask;
+
+  uint32_t bx, by, ox, oy, width, height, sub;  // sub-block and tile origin, the view's size
+  size_t pix0;                                  // the view's first pixel
+  uint2 range;                                  // the tile's entries
+  const uint32_t* gauss;
+  const float4* rec;
+
+  // Sub-block of warp `w` of the grid; false past the last tile (then for all its warps). A
+  // batch numbers its tiles across the views.
+  __device__ __forceinline__ bool init(uint32_t w, uint32_t tiles, uint32_t width_, uint32_t height_,
+                                       uint32_t tiles_x, const uint32_t* __restrict__ gauss_,
+                                       const float4* __restrict__ rec_, const uint2* __restrict__ ranges,
+                                       const BatchTable* __restrict__ bt) {
+    const uint32_t global = w / kPerTile;
+    sub = w % kPerTile;
+    if (global >= (bt ? bt->tile_start[bt->views] : tiles)) return false;
+    uint32_t tile = global;
+    pix0 = 0;
+    width = width_;
+    height = height_;
+    if (bt) {
+      const int v = batch_view_of(bt->tile_start, bt->views, global);
+      tile = global - bt->tile_start[v];
+      width = bt->cam[v].width;
+      height = bt->cam[v].height;
+      tiles_x = bt->tiles_x[v];
+      pix0 = bt->pix_start[v];
     }
-    __syncthreads();
-    const uint32_t cnt = min((uint32_t)CH, range.y - base);
-    const uint32_t nl = build_warp_list(smask, cnt, 0xffffffffu, list);
-    for (uint32_t b0 = 0; b0 < nl; b0 += 32) {
-      if (__all_sync(0xffffffffu, done)) break;
-      // Lane j loads entry j of the batch and expands its rectangle to a 32-bit mask of the
-      // sub-block's pixels (bit 8 * row + column); the transpose gives each lane the mask of
-      // the batch entries that cover its pixel.
-      const uint32_t j = b0 + lane;
-      uint32_t kl = 0, cov = 0;
-      if (j < nl) {
-        kl = list[j];
-        const typename Geo::Mask rm = srect[kl];
-        const uint32_t c8 = (uint32_t)(rm >> sbx) & 0xffu;
-        const uint32_t r4 = (uint32_t)(rm >> sby) & 0xfu;
-        cov = c8 * ((r4 & 1u) | ((r4 & 2u) << 7) | ((r4 & 4u) << 14) | ((r4 & 8u) << 21));
+    ox = (tile % tiles_x) * TW;
+    oy = (tile / tiles_x) * TH;
+    bx = ox + (sub % kAcross) * 8u;
+    by = oy + (sub / kAcross) * BH;
+    range = ranges[global];
+    gauss = gauss_ + range.x;
+    rec = rec_;
+    return true;
+  }
+
+  // Barrier over the tile's warps; a block holds `kTiles` tiles, each with a barrier of its own.
+  template <int kTiles>
+  __device__ __forceinline__ void barrier() const {
+    if (kPerTile == 1) {
+      __syncwarp();
+    } else if (kTiles == 1) {
+      __syncthreads();
+    } else {
+      const uint32_t id = 1u + (threadIdx.x >> 5) / kPerTile;
+      asm volatile("barrier.cta.sync %0, %1;" ::"r"(id), "n"(32 * kPerTile) : "memory");
+    }
+  }
+  // The same; true when `p` holds in every thread of the tile's warps.
+  template <int kTiles>
+  __device__ __forceinline__ bool barrier_all(bool p) const {
+    if (kPerTile == 1) return __all_sync(0xffffffffu, p);
+    if (kTiles == 1) return __syncthreads_and(p);
+    const uint32_t id = 1u + (threadIdx.x >> 5) / kPerTile;
+    uint32_t r;
+    asm volatile(
+        "{\n.reg .pred p, q;\nsetp.ne.u32 p, %1, 0;\nbarrier.cta.red.and.pred q, %2, %3, p;\nselp.u32 %0, 1, 0, q;\n}"
+        : "=r"(r)
+        : "r"((uint32_t)p), "r"(id), "n"(32 * kPerTile)
+        : "memory");
+    return r != 0;
+  }
+
+  // The tile's warps scan list entries first, first + step, ... (`cnt` of them, step 1 or -1)
+  // into `list`: each entry's rectangle is loaded once for the whole tile.
+  __device__ __forceinline__ void scan(TileList<Mask>& list, uint32_t first, int step, uint32_t cnt) const {
+    constexpr uint32_t kThreads = 32 * kPerTile, kBatch = kPerTile >= 8 ? kListChunk / kThreads : 4;
+    const uint32_t t = sub * 32u + (threadIdx.x & 31u);
+    for (uint32_t i0 = t; i0 < cnt; i0 += kThreads * kBatch) {
+      uint32_t g[kBatch];
+      float2 r[kBatch];
+#pragma unroll
+      for (uint32_t q = 0; q < kBatch; q++) {
+        const uint32_t i = i0 + q * kThreads;
+        g[q] = i < cnt ? gauss[first + (uint32_t)(step * (int)i)] : 0u;
       }
+#pragma unroll
+      for (uint32_t q = 0; q < kBatch; q++)
+        if (i0 + q * kThreads < cnt) r[q] = reinterpret_cast<const float2*>(rec + 4 * (size_t)g[q] + 2)[1];
+#pragma unroll
+      for (uint32_t q = 0; q < kBatch; q++) {
+        const uint32_t i = i0 + q * kThreads;
+        if (i < cnt) {
+          list.g[i] = g[q];
+          list.mask[i] = (Mask)subblock_mask<TW, TH, BH>(fbits(r[q].x), fbits(r[q].y), ox, oy);
+        }
+      }
+    }
+  }
+};
+
+__device__ __forceinline__ void copy_async16(float4* smem, const float4* global) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(d), "l"(global) : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// One warp's pass over a scanned list: the entries whose mask has the warp's bit, in order,
+// queued (as list indices) and staged 32 at a time.
+template <typename Mask>
+struct Stager {
+  const TileList<Mask>* list;
+  uint32_t cnt, pos, head, tail, bit;
+  uint16_t* queue;
+  __device__ __forceinline__ void start(const TileList<Mask>* l, uint32_t cnt_, uint32_t bit_, uint16_t* q) {
+    list = l;
+    cnt = cnt_;
+    bit = bit_;
+    queue = q;
+    pos = head = tail = 0;
+  }
+  // Starts the copies of the next stage's records, part p of entry i to s + p * stride + i
+  // (four lanes per record: one 64-byte line each); returns how many entries, and through *g
+  // and *index this lane's Gaussian and list index.
+  __device__ __forceinline__ uint32_t fetch(const float4* __restrict__ rec, float4* s, uint32_t stride, uint32_t* g,
+                                            uint32_t* index) {
+    const uint32_t lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
+    while (tail - head < (uint32_t)kStage && pos < cnt) {
+      const uint32_t i = pos + lane;
+      const bool hit = i < cnt && ((list->mask[i] >> bit) & 1u);
+      const uint32_t bal = __ballot_sync(0xffffffffu, hit);
+      if (hit) queue[(tail + __popc(bal & lt)) & (kQueue - 1)] = (uint16_t)i;
+      tail += __popc(bal);
+      pos += 32u;
+    }
+    __syncwarp();
+    const uint32_t m = min(tail - head, (uint32_t)kStage);
+    if (lane < m) {
+      *index = queue[(head + lane) & (kQueue - 1)];
+      *g = list->g[*index];
+    }
+    const uint32_t part = lane & 3u;
+#pragma unroll
+    for (uint32_t q = 0; q < 4; q++) {
+      const uint32_t i = 8u * q + (lane >> 2);
+      const uint32_t gi = __shfl_sync(0xffffffffu, *g, i);
+      if (i < m && part < 3u) copy_async16(s + part * stride + i, rec + 4 * (size_t)gi + part);
+    }
+    head += m;
+    __syncwarp();
+    return m;
+  }
+};
+
+// 32x32 bit-matrix transpose across a warp: lane j holds row j on entry; on return lane L
+// holds column L (bit j of the result = bit L of lane j's input). Five exchange stages,
+// each swapping the off-diagonal blocks of size s.
+__device__ __forceinline__ uint32_t warp_transpose_bits(uint32_t x) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t masks[5] = {0x0000ffffu, 0x00ff00ffu, 0x0f0f0f0fu, 0x33333333u, 0x55555555u};
+#pragma unroll
+  for (int i = 0; i < 5; i++) {
+    const uint32_t sh = 16u >> i, m = masks[i];
+    const uint32_t y = __shfl_xor_sync(0xffffffffu, x, sh);
+    x = (lane & sh) ? ((x & ~m) | ((y & ~m) >> sh)) : ((x & m) | ((y & m) << sh));
+  }
+  return x;
+}
+
+// Columns (bits 0-7) and rows (bits 8-15) of the 8 x 8 block at (bx, by) inside the pixel
+// rectangle (x0|x1<<16, y0|y1<<16); 0 in either half when it is empty.
+__device__ __forceinline__ uint32_t sub_block_mask(uint32_t rx, uint32_t ry, uint32_t bx, uint32_t by) {
+  const int x0 = min(max((int)(rx & 0xffffu) - (int)bx, 0), 8), x1 = min(max((int)(rx >> 16) - (int)bx, 0), 8);
+  const int y0 = min(max((int)(ry & 0xffffu) - (int)by, 0), 8), y1 = min(max((int)(ry >> 16) - (int)by, 0), 8);
+  const uint32_t cols = ((1u << x1) - 1u) & ~((1u << x0) - 1u);
+  const uint32_t rows = ((1u << y1) - 1u) & ~((1u << y0) - 1u);
+  return cols | (rows << 8);
+}
+
+// An entry whose sigma could overflow to inf or NaN, whose sigma_max passes the exp table or
+// whose colour or opacity is not finite (none of which a projection of finite parameters
+// gives) is composited by the scalar path.
+__device__ __forceinline__ bool special_entry(float4 r0, float4 r1, float4 r2) {
+  const bool plain = fabsf(r0.x) < 1e9f && fabsf(r0.y) < 1e9f && fabsf(r0.z) < 1e15f && fabsf(r0.w) < 1e15f &&
+                     fabsf(r1.x) < 1e15f && fabsf(r1.y) < 1e15f && r1.z <= crm::kExpGridMax && fabsf(r1.w) < 1e30f &&
+                     fabsf(r2.x) < 1e30f && fabsf(r2.y) < 1e30f;
+  return !plain;
+}
+
+// forward_tile (rasterize.rs:249-302): each warp composites an 8x4 sub-block, one pixel per
+// lane, entries in list (depth) order. For every 32 staged entries the coverage masks
+// (lane j: the sub-block's pixels inside entry j's rectangle) are transposed across the warp,
+// and each lane then walks only the entries that cover its own pixel, so the warp runs as
+// many rounds as its busiest lane. A round has no branch on the decisions: a lane out of
+// entries takes the null entry (index kStage), a pixel that skips its entry takes alpha = 0,
+// which leaves transmittance and colour exactly as they are. exp is the correctly rounded one
+// (crm::expf_cr_grid; its table in shared memory, six double operations). kCount adds the
+// evaluated-pair counter (untimed diagnostics only).
+// Bound by instruction issue (73%) and shared-memory reads (62%: divergent 16-byte record
+// reads and the exp table). Time against one block per tile staging chunks between barriers,
+// with a 577-entry exp table and its rounding in double: 1M Gaussians at 1920x1080 542 ->
+// 428 us, 187k clustered at 1297x840 264 -> 194, 34k at 256x256 86 -> 53. 32 warps per SM (64
+// registers) beat 40 (spills; 432, 199 and 60 us). A pixel pair per lane in f32x2 arithmetic
+// with every lane on the same entry was slower on small Gaussians (616 us) and at 256x256.
+struct FwdStage {
+  float4 s[2][3][kStage + 1];  // records (three of their four quads), double-buffered; the last entry is null
+  uint16_t queue[kQueue];
+};
+template <int TW, int TH>
+struct FwdShape {
+  typedef Walk<TW, TH, 4> W;
+  static constexpr int kWarps = W::kPerTile > 8 ? W::kPerTile : 8, kTiles = kWarps / W::kPerTile;
+};
+template <int TW, int TH>
+struct FwdSmem {
+  double tab[crm::kExpGridEntries];
+  FwdStage stage[FwdShape<TW, TH>::kWarps];
+  TileList<typename Walk<TW, TH, 4>::Mask> list[FwdShape<TW, TH>::kTiles];
+};
+
+__device__ const crm::ExpGrid kExpGrid{};
+
+template <int TW, int TH, bool kCount>
+__global__ void __launch_bounds__(32 * FwdShape<TW, TH>::kWarps, 32 / FwdShape<TW, TH>::kWarps) raster_fwd_kernel(
+    const float4* __restrict__ rec, const uint32_t* __restrict__ gauss, const uint2* __restrict__ ranges,
+    uint32_t tiles, uint32_t width, uint32_t height, uint32_t tiles_x, float bg0, float bg1, float bg2,
+    float* __restrict__ image, float* __restrict__ final_t, uint32_t* __restrict__ n_contrib,
+    unsigned long long* __restrict__ pairs, const BatchTable* __restrict__ bt) {
+  typedef FwdShape<TW, TH> Shape;
+  typedef typename Shape::W W;
+  extern __shared__ __align__(16) unsigned char raster_smem[];
+  FwdSmem<TW, TH>& sm = *reinterpret_cast<FwdSmem<TW, TH>*>(raster_smem);
+  for (int i = threadIdx.x; i < crm::kExpGridEntries; i += 32 * Shape::kWarps) sm.tab[i] = kExpGrid.v[i];
+  __syncthreads();
+  const double* tab = sm.tab;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  W wk;
+  if (!wk.init(blockIdx.x * Shape::kWarps + warp, tiles, width, height, tiles_x, gauss, rec, ranges, bt)) return;
+  FwdStage& st = sm.stage[warp];
+  TileList<typename W::Mask>& list = sm.list[warp / W::kPerTile];
+  if (lane < 2) {
+    st.s[lane][0][kStage] = st.s[lane][2][kStage] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    st.s[lane][1][kStage] = make_float4(0.0f, 0.0f, -1.0f, 0.0f);  // sigma_max < 0: never taken
+  }
+  const uint32_t x = wk.bx + (lane & 7u), y = wk.by + (lane >> 3);
+  const bool inside = x < wk.width && y < wk.height;
+  const float px = (float)x + 0.5f, py = (float)y + 0.5f;
+  float T = 1.0f, cr = 0.0f, cg = 0.0f, cb = 0.0f;
+  uint32_t ncon = 0, npairs = 0;
+  bool done = !inside;
+
+  const uint32_t n = wk.range.y - wk.range.x;
+  for (uint32_t first = 0; first < n; first += kListChunk) {
+    if (first && wk.template barrier_all<Shape::kTiles>(done)) break;
+    const uint32_t cnt = min(n - first, (uint32_t)kListChunk);
+    wk.scan(list, first, 1, cnt);
+    wk.template barrier<Shape::kTiles>();
+    if (__all_sync(0xffffffffu, done)) continue;
+    Stager<typename W::Mask> stager;
+    stager.start(&list, cnt, wk.sub, st.queue);
+    uint32_t buf = 0, g = 0, index = 0;
+    uint32_t m = stager.fetch(rec, st.s[0][0], kStage + 1, &g, &index);
+    while (m) {
+      copy_async_wait();
+      __syncwarp();
+      const float4* s0 = st.s[buf][0];
+      const float4* s1 = st.s[buf][1];
+      const float4* s2 = st.s[buf][2];
+      uint32_t cov = 0;
+      bool special = false;
+      if (lane < m) {
+        const float4 r2 = s2[lane];
+        const uint32_t mask = sub_block_mask(fbits(r2.z), fbits(r2.w), wk.bx, wk.by);
+        const uint32_t r4 = (mask >> 8) & 0xfu;
+        cov = (mask & 0xffu) * ((r4 & 1u) | ((r4 & 2u) << 7) | ((r4 & 4u) << 14) | ((r4 & 8u) << 21));
+        special = special_entry(s0[lane], s1[lane], r2);
+      }
+      const uint32_t place = first + index + 1u;  // n_contrib of a pixel whose last entry is this lane's
+      special = __any_sync(0xffffffffu, special);
       uint32_t mine = warp_transpose_bits(cov);
       if (done) mine = 0;
-      while (__any_sync(0xffffffffu, mine != 0u)) {
-        const uint32_t k = __shfl_sync(0xffffffffu, kl, (__ffs(mine) - 1) & 31);
-        if (mine == 0u) continue;
-        mine &= mine - 1u;
-        if (kCount) npairs++;
-        const float4 e0 = s0[k], e1 = s1[k];
-        const float2 e2 = s2[k];
-        float gval, alpha;
-        if (!evaluate(px, py, e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, stab, &gval, &alpha)) continue;
-        const float test_t = T * (1.0f - alpha);
-        if (test_t < SPLAT_T_MIN) {
-          done = true;
-          mine = 0;
-          continue;
+      buf ^= 1u;
+      m = stager.fetch(rec, st.s[buf][0], kStage + 1, &g, &index);  // loads while this stage is composited
+      if (kCount) npairs += __popc(mine);
+      uint32_t taken = kStage;  // the stage's last entry this pixel took
+      if (!special) {
+        while (__any_sync(0xffffffffu, mine != 0u)) {
+          const uint32_t k = mine ? (uint32_t)__ffs((int)mine) - 1u : (uint32_t)kStage;
+          mine &= mine - 1u;
+          const float4 e0 = s0[k], e1 = s1[k];
+          const float2 e2 = *reinterpret_cast<const float2*>(s2 + k);
+          const float dx = px - e0.x, dy = py - e0.y;
+          const float sigma = 0.5f * (e0.z * dx * dx + e1.x * dy * dy) + e0.w * dx * dy;
+          const bool in = sigma >= 0.0f && sigma <= e1.z;
+          const float sg = in ? sigma : crm::kExpGridSkip;
+          const float mm = __fmaf_rn(sg, 128.0f, crm::kExpGridMagic);
+          const float t = __fmaf_rn(mm - crm::kExpGridMagic, -0.0078125f, sg);
+          const float og = e1.y * crm::exp_grid_finish(t, tab[fbits(mm) & 1023u]);
+          float alpha = og < SPLAT_ALPHA_MIN ? 0.0f : fminf(og, SPLAT_ALPHA_MAX);
+          float test_t = T * (1.0f - alpha);
+          if (test_t < SPLAT_T_MIN) {  // the pixel is done without this entry
+            if (kCount) npairs -= __popc(mine);
+            done = true;
+            mine = 0;
+            alpha = 0.0f;
+            test_t = T;
+          }
+          const float at = alpha * T;
+          cr += at * e1.w;
+          cg += at * e2.x;
+          cb += at * e2.y;
+          T = test_t;
+          taken = alpha > 0.0f ? k : taken;
         }
-        const float at = alpha * T;
-        cr += at * e1.w;
-        cg += at * e2.x;
-        cb += at * e2.y;
-        T = test_t;
-        ncon = base - range.x + k + 1;
+      } else {
+        while (mine) {
+          const uint32_t k = (uint32_t)__ffs((int)mine) - 1u;
+          mine &= mine - 1u;
+          const float4 e0 = s0[k], e1 = s1[k], e2 = s2[k];
+          float gval, alpha;
+          if (!evaluate_ref(px, py, e0.x, e0.y, e0.z, e0.w, e1.x, e1.y, e1.z, &gval, &alpha)) continue;
+          const float test_t = T * (1.0f - alpha);
+          if (test_t < SPLAT_T_MIN) {
+            if (kCount) npairs -= __popc(mine);
+            done = true;
+            break;
+          }
+          const float at = alpha * T;
+          cr += at * e1.w;
+          cg += at * e2.x;
+          cb += at * e2.y;
+          T = test_t;
+          taken = k;
+        }
       }
+      const uint32_t last_place = __shfl_sync(0xffffffffu, place, taken & 31u);
+      if (taken < (uint32_t)kStage) ncon = last_place;
+      if (__all_sync(0xffffffffu, done)) break;
     }
-    __syncthreads();
+    copy_async_wait();  // copies may be in flight past an early stop
+    __syncwarp();
   }
-  if (pg.inside) {
-    const size_t pix = pix0 + (size_t)pg.py_j * width + pg.px_i;
+  if (inside) {
+    const size_t pix = wk.pix0 + (size_t)y * wk.width + x;
     image[3 * pix] = cr + T * bg0;
     image[3 * pix + 1] = cg + T * bg1;
     image[3 * pix + 2] = cb + T * bg2;
@@ -418,8 +615,9 @@ __global__ void __launch_bounds__(TW * TH, 1536 / (TW * TH)) raster_fwd_kernel(
     n_contrib[pix] = ncon;
   }
   if (kCount) {
-    for (int o = 16; o > 0; o >>= 1) npairs += __shfl_xor_sync(0xffffffffu, npairs, o);
-    if (lane == 0 && npairs) atomicAdd(pairs, npairs);
+    unsigned long long np = npairs;
+    for (int o = 16; o > 0; o >>= 1) np += __shfl_xor_sync(0xffffffffu, np, o);
+    if (lane == 0 && np) atomicAdd(pairs, np);
   }
 }
 
@@ -681,80 +879,187 @@ __global__ void __launch_bounds__(TW * TH / PPL, (PPL == 1 ? 1024 : 768) / (TW *
 // fl(opacity * exp(-sigma)) <= opacity, so an entry with opacity < 0.99 never clamps.
 constexpr float kSigmaEdge = 1e-4f;
 
-// The backward with two pixels per thread computed as pairs. Lane L owns the pixels
-// (L % 8, L / 8) and (L % 8, L / 8 + 4) of its warp's 8x8 sub-block; every per-pixel value of
-// backward_tile (rasterize.rs:394-454) is a pair, computed with the paired instructions of
-// pair.cuh, and an entry's record is staged in shared memory with each scalar duplicated
-// into both halves so that it is an operand as it stands. Decisions are taken on the
-// halves: sigma (bit-identical to the scalar sigma) against the entry's range, as above.
-// A pixel the entry does not reach (outside the rectangle, at or past n_contrib, skipped by
-// a decision) runs the arithmetic with sigma = +inf, so gauss = alpha = 0: its
-// transmittance is multiplied by rcp(1) = 1 exactly, its colour accumulator by 0 + 1, and
-// all its contributions are exactly zero; both pixels of a pair always run together and
-// still leave the scalar kernel's state and sums. The colour accumulator is advanced right
-// after its use (accum + alpha (c - accum)) instead of on the pixel's next entry, which
-// needs the same operands and so leaves neither last_alpha nor last_color to carry. A
-// lane's two contributions to each slot are added before the warp reduction. kCount adds
-// the evaluated-pair counter (untimed diagnostics only).
-template <int TW, int TH, int CH, bool kCount>
-__global__ void __launch_bounds__(TW * TH / 2, 768 / (TW * TH / 2)) raster_bwd_x2_kernel(
+// The backward with two pixels per thread computed as pairs, each warp alone on an 8x8
+// sub-block (lane L owns the pixels (L % 8, L / 8) and (L % 8, L / 8 + 4)), in two phases.
+//
+// Phase A walks the staged entries in reverse depth order, a pixel pair per lane: every
+// per-pixel value of backward_tile (rasterize.rs:394-454) is a pair, computed with the paired
+// instructions of pair.cuh from records staged with each scalar duplicated. Decisions are
+// taken on the halves: sigma (bit-identical to the scalar sigma) against the entry's range,
+// as above. A pixel the entry does not reach (outside the rectangle, at or past n_contrib,
+// skipped by a decision) runs the arithmetic with sigma = +inf, so gauss = alpha = 0: its
+// transmittance is multiplied by rcp(1) = 1 exactly, its colour accumulator by 0 + 1, and all
+// its contributions are exactly zero. The colour accumulator is advanced right after its use
+// (accum + alpha (c - accum)), which needs the same operands as the reference's lazy update.
+// What a pixel contributes to the entry's gradients is two numbers: h = gauss dL/dalpha and
+// w = alpha T. Each taken entry leaves the sub-block's 64 pairs (h, w) in one of kGroup rows
+// of shared memory.
+//
+// Phase B runs when kGroup rows are full: lane L takes entry L % 8 and the rows L / 8 and
+// L / 8 + 4 of the sub-block, i.e. 16 of the entry's pixels, and sums h {1, dx, dx^2} (dy and
+// its products are constant over a row), w {1, dL/dr, dL/dg, dL/db} and the two absolute
+// gradients over them; the 12 slots follow by linear combination (with -dsigma = opacity h)
+// and two exchange stages add the four lanes of an entry. This replaces 12 per-lane products
+// and a 13-shuffle reduction over the warp for every entry: per entry about 35 warp
+// instructions instead of 95 (1M Gaussians at 1920x1080: 975 -> 794 us; 187k clustered at 1297x840:
+// 377 -> 300). The entry's sums go from here to global memory with one float4
+// vector atomic per gradient plane.
+// kCount adds the evaluated-pair counter (untimed diagnostics only).
+constexpr int kGroup = 8;
+constexpr int kGroupRow = 33;  // float4 per row: 32 lanes and a pad, so that 8 rows hit distinct banks
+struct BwdStage {
+  // Staged entries: (mx mx my my), (A A B B), (C C opacity sigma_max), (r r g g), (b b, coverage
+  // mask, list position), Gaussian.
+  float4 xy[kStage], ab[kStage], co[kStage], rg[kStage], bm[kStage];
+  uint32_t g[kStage];
+  float4 s[3][kStage];  // the next stage's records as they arrive
+  uint16_t queue[kQueue];
+  float4 hw[kGroup * kGroupRow];  // (h, h, w, w) of a lane's pixel pair
+  float4 d01[32];                 // dL/dr and dL/dg of a lane's pair
+  float2 d2[32];                  // dL/db
+};
+
+template <int TW, int TH>
+struct BwdShape {
+  typedef Walk<TW, TH, 8> W;
+  static constexpr int kWarps = W::kPerTile > 4 ? W::kPerTile : 4, kTiles = kWarps / W::kPerTile;
+};
+template <int TW, int TH>
+struct BwdSmem {
+  BwdStage stage[BwdShape<TW, TH>::kWarps];
+  TileList<typename Walk<TW, TH, 8>::Mask> list[BwdShape<TW, TH>::kTiles];
+  uint32_t max_last[BwdShape<TW, TH>::kTiles];
+};
+
+// Coverage word of a lane's pixel (column c, row r of the sub-block): the pixel is covered
+// when the entry's mask has both its bits.
+__device__ __forceinline__ uint32_t pixel_bits(uint32_t c, uint32_t r) { return (1u << c) | (256u << r); }
+
+// Phase B: lane `lane` sums entry `lane % 8` of the group (staged index kk, `count` rows
+// valid) over the rows of the sub-block whose first pixel centre is (px0, py0) and adds the
+// 12 slots to pgrad.
+__device__ __forceinline__ void reduce_group(BwdStage& st, uint32_t count, uint32_t kk, float px0, float py0,
+                                             float4* __restrict__ pgrad, int64_t cap) {
+  const uint32_t lane = threadIdx.x & 31, e = lane & 7u, q = lane >> 3;
+  const float4 exy = st.xy[kk], eab = st.ab[kk], eco = st.co[kk];
+  const float my = exy.z;
+  const f2 A = f2_make(eab.x, eab.y), B = f2_make(eab.z, eab.w);
+  const float dy0 = (py0 + (float)q) - my, dy1 = (py0 + (float)(q + 4u)) - my;
+  const f2 dy = f2_make(dy0, dy1);
+  const f2 bdy = f2_mul(B, dy), cdy = f2_mul(f2_make(eco.x, eco.y), dy);
+  const f2 dx0 = f2_splat(px0 - exy.x);
+  f2 h0 = f2_splat(0.0f), h1 = h0, h2 = h0, w0 = h0, wr = h0, wg = h0, wb = h0;
+  float ax = 0.0f, ay = 0.0f;
+#pragma unroll
+  for (int c = 0; c < 8; c++) {
+    const float4 v = st.hw[e * kGroupRow + q * 8u + c];
+    const float4 d01 = st.d01[q * 8u + c];
+    const float2 d2 = st.d2[q * 8u + c];
+    const f2 h = f2_make(v.x, v.y), w = f2_make(v.z, v.w);
+    const f2 dx = c == 0 ? dx0 : f2_add(dx0, f2_splat((float)c));
+    const f2 hx = f2_mul(h, dx);
+    h0 = f2_add(h0, h);
+    h1 = f2_add(h1, hx);
+    h2 = f2_fma(hx, dx, h2);
+    w0 = f2_add(w0, w);
+    wr = f2_fma(w, f2_make(d01.x, d01.y), wr);
+    wg = f2_fma(w, f2_make(d01.z, d01.w), wg);
+    wb = f2_fma(w, f2_make(d2.x, d2.y), wb);
+    float lo, hi;
+    f2_split(f2_mul(h, f2_fma(A, dx, bdy)), lo, hi);
+    ax += fabsf(lo);
+    ax += fabsf(hi);
+    f2_split(f2_mul(h, f2_fma(B, dx, cdy)), lo, hi);
+    ay += fabsf(lo);
+    ay += fabsf(hi);
+  }
+  // Slots 0-11: d mean2d.x, .y, d conic A, B, C, d opacity, d r, g, b, |d mean2d.x|, |.y|, sum(alpha T).
+  float v[kSlots], lo, hi;
+  const float op = eco.z;
+  f2_split(h0, lo, hi);
+  const float sy = __fmaf_rn(dy1, hi, dy0 * lo), syy = __fmaf_rn(dy1 * dy1, hi, (dy0 * dy0) * lo);
+  v[5] = lo + hi;
+  f2_split(h1, lo, hi);
+  const float sx = lo + hi, sxy = __fmaf_rn(dy1, hi, dy0 * lo);
+  f2_split(h2, lo, hi);
+  const float sxx = lo + hi;
+  v[0] = op * __fmaf_rn(eab.x, sx, eab.z * sy);
+  v[1] = op * __fmaf_rn(eab.z, sx, eco.x * sy);
+  v[2] = -0.5f * op * sxx;
+  v[3] = -op * sxy;
+  v[4] = -0.5f * op * syy;
+  f2_split(wr, lo, hi);
+  v[6] = lo + hi;
+  f2_split(wg, lo, hi);
+  v[7] = lo + hi;
+  f2_split(wb, lo, hi);
+  v[8] = lo + hi;
+  v[9] = fabsf(op) * ax;
+  v[10] = fabsf(op) * ay;
+  f2_split(w0, lo, hi);
+  v[11] = lo + hi;
+  // Two exchange stages over the entry's four lanes: 6 + 3 shuffles leave lane (e, q) with
+  // slots 3 q .. 3 q + 2 (q's bit 1 chooses the half, bit 0 the half of the half).
+  const bool b1 = lane & 16u, b0 = lane & 8u;
+  float x6[6], x3[3];
+#pragma unroll
+  for (int i = 0; i < 6; i++) x6[i] = (b1 ? v[i + 6] : v[i]) + __shfl_xor_sync(0xffffffffu, b1 ? v[i] : v[i + 6], 16);
+#pragma unroll
+  for (int i = 0; i < 3; i++) x3[i] = (b0 ? x6[i + 3] : x6[i]) + __shfl_xor_sync(0xffffffffu, b0 ? x6[i] : x6[i + 3], 8);
+  __syncwarp();  // every lane has read the rows: they take the sums
+  float* out = reinterpret_cast<float*>(st.hw);
+#pragma unroll
+  for (int i = 0; i < 3; i++) out[e * kSlots + 3u * q + i] = x3[i];
+  __syncwarp();
+  const uint32_t i = lane / 3u, p = lane - 3u * i;  // lane 3 i + p: plane p of entry i
+  const uint32_t ki = __shfl_sync(0xffffffffu, kk, i & 7u);
+  if (i < count) {
+    const float4 t = st.hw[lane];
+    if (t.x != 0.0f || t.y != 0.0f || t.z != 0.0f || t.w != 0.0f) atomicAdd(&pgrad[p * (size_t)cap + st.g[ki]], t);
+  }
+  __syncwarp();
+}
+
+template <int TW, int TH, bool kCount>
+__global__ void __launch_bounds__(32 * BwdShape<TW, TH>::kWarps, 16 / BwdShape<TW, TH>::kWarps) raster_bwd_x2_kernel(
     const float4* __restrict__ rec, const uint32_t* __restrict__ gauss, const uint2* __restrict__ ranges,
-    uint32_t width, uint32_t height, uint32_t tiles_x, float bg0, float bg1, float bg2,
+    uint32_t tiles, uint32_t width, uint32_t height, uint32_t tiles_x, float bg0, float bg1, float bg2,
     const float* __restrict__ final_t, const uint32_t* __restrict__ n_contrib, const float* __restrict__ dimage,
     float4* __restrict__ pgrad, int64_t cap, unsigned long long* __restrict__ pairs,
     const BatchTable* __restrict__ bt) {
-  typedef TileGeo<TW, TH> Geo;
-  typedef typename Geo::Mask Mask;
-  constexpr int NT = TW * TH / 2, NW = NT / 32, WX = TW / 8, SBH = 8;
-  typedef typename std::conditional<(NW > 8), uint16_t, uint8_t>::type WarpMask;
-  if (bt && blockIdx.x >= bt->tile_start[bt->views]) return;  // past the batch's tiles
-  // Per entry, duplicated: (mx, mx, my, my), (A, A, B, B), (C, C, opacity, opacity),
-  // (r, r, g, g), (b, b); and (sigma_max, sigma_max - kSigmaEdge).
-  __shared__ float4 sxy[CH], sab[CH], sco[CH], srg[CH];
-  __shared__ float2 sb[CH], ssig[CH];
-  __shared__ Mask srect[CH];
-  __shared__ uint32_t sg[CH];
-  __shared__ float acc[CH * kSlots];
-  __shared__ WarpMask smask[CH];
-  __shared__ uint8_t slist[NW][CH];
-  __shared__ uint32_t s_max_last;
-  uint32_t tile = blockIdx.x;
-  size_t pix0 = 0;
-  if (bt) {
-    const int v = batch_view_of(bt->tile_start, bt->views, blockIdx.x);
-    tile = blockIdx.x - bt->tile_start[v];
-    width = bt->cam[v].width;
-    height = bt->cam[v].height;
-    tiles_x = bt->tiles_x[v];
-    pix0 = bt->pix_start[v];
-  }
-  const uint32_t ox = (tile % tiles_x) * TW, oy = (tile / tiles_x) * TH;
+  typedef BwdShape<TW, TH> Shape;
+  typedef typename Shape::W W;
+  extern __shared__ __align__(16) unsigned char raster_smem[];
+  BwdSmem<TW, TH>& sm = *reinterpret_cast<BwdSmem<TW, TH>*>(raster_smem);
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t lx = (warp % WX) * 8u + (lane & 7u);
-  const uint32_t ly0 = (warp / WX) * (uint32_t)SBH + (lane >> 3);
-  // A pixel is in an entry's rectangle when both its column and its row bit are set.
-  const Mask bits0 = ((Mask)1 << lx) | ((Mask)1 << (ly0 + Geo::kRowShift));
-  const Mask bits1 = ((Mask)1 << lx) | ((Mask)1 << (ly0 + 4u + Geo::kRowShift));
-  const uint2 range = ranges[blockIdx.x];
-  uint8_t* list = slist[warp];
-  const uint32_t list_len = range.y - range.x;
+  W wk;
+  if (!wk.init(blockIdx.x * Shape::kWarps + warp, tiles, width, height, tiles_x, gauss, rec, ranges, bt)) return;
+  BwdStage& st = sm.stage[warp];
+  TileList<typename W::Mask>& list = sm.list[warp / W::kPerTile];
+  uint32_t& tile_last = sm.max_last[warp / W::kPerTile];
+  if (wk.sub == 0 && lane == 0) tile_last = 0;
+  wk.template barrier<Shape::kTiles>();
+  const uint32_t col = lane & 7u, row = lane >> 3;
+  const uint32_t bits0 = pixel_bits(col, row), bits1 = pixel_bits(col, row + 4u);
+  const uint32_t list_len = wk.range.y - wk.range.x;
 
   // Per pixel pair: pixel centres, contributor counts, transmittance, dL/dpixel, the
   // background's share of dL/dalpha (times 1 - alpha) and the colour accumulator.
-  const float pxf = (float)(ox + lx) + 0.5f;
-  const f2 px = f2_splat(pxf);
-  const f2 py = f2_make((float)(oy + ly0) + 0.5f, (float)(oy + ly0 + 4u) + 0.5f);
+  const uint32_t x = wk.bx + col;
+  const float px0 = (float)wk.bx + 0.5f, py0 = (float)wk.by + 0.5f;
+  const f2 px = f2_splat((float)x + 0.5f);
+  const f2 py = f2_make((float)(wk.by + row) + 0.5f, (float)(wk.by + row + 4u) + 0.5f);
   uint32_t last[2];
   float Tq[2], nbgq[2], d0q[2], d1q[2], d2q[2];
 #pragma unroll
   for (int q = 0; q < 2; q++) {
-    const uint32_t y = oy + ly0 + 4u * q, x = ox + lx;
+    const uint32_t y = wk.by + row + 4u * q;
     last[q] = 0;
     Tq[q] = 1.0f;
     d0q[q] = d1q[q] = d2q[q] = nbgq[q] = 0.0f;
-    if (x < width && y < height) {
-      const size_t pix = pix0 + (size_t)y * width + x;
-      last[q] = min(n_contrib[pix], list_len);
+    if (x < wk.width && y < wk.height) {
+      const size_t pix = wk.pix0 + (size_t)y * wk.width + x;
+      last[q] = min(n_contrib[pix], list_len);  // n_contrib never exceeds its tile's list
       Tq[q] = final_t[pix];
       d0q[q] = dimage[3 * pix];
       d1q[q] = dimage[3 * pix + 1];
@@ -766,162 +1071,113 @@ __global__ void __launch_bounds__(TW * TH / 2, 768 / (TW * TH / 2)) raster_bwd_x
   const f2 nbg = f2_make(nbgq[0], nbgq[1]);
   const f2 d0 = f2_make(d0q[0], d0q[1]), d1 = f2_make(d1q[0], d1q[1]), d2 = f2_make(d2q[0], d2q[1]);
   f2 acc_r = f2_splat(0.0f), acc_g = acc_r, acc_b = acc_r;
-  const f2 half = f2_splat(0.5f), one = f2_splat(1.0f), nlog2e = f2_splat(-kLog2e);
-  const uint32_t lane_last = max(last[0], last[1]);
+  const f2 one = f2_splat(1.0f), nlog2e = f2_splat(-kLog2e);
+  st.d01[lane] = make_float4(d0q[0], d0q[1], d1q[0], d1q[1]);
+  st.d2[lane] = make_float2(d2q[0], d2q[1]);
+  uint32_t npairs = 0, count = 0, mykk = 0;
 
-  if (threadIdx.x == 0) s_max_last = 0;
-  for (int i = threadIdx.x; i < CH * kSlots; i += NT) acc[i] = 0.0f;
-  __syncthreads();
-  const uint32_t warp_max_last = __reduce_max_sync(0xffffffffu, lane_last);
-  if (lane == 0) atomicMax(&s_max_last, warp_max_last);
-  __syncthreads();
-  const uint32_t max_last = s_max_last;
-  uint32_t npairs = 0;
-
-  for (uint32_t cend = max_last; cend > 0;) {
-    const uint32_t cstart = cend > (uint32_t)CH ? cend - CH : 0u;
-    const uint32_t cnt = cend - cstart;
-#pragma unroll
-    for (uint32_t e = threadIdx.x; e < (uint32_t)CH; e += NT) {
-      uint32_t m = 0;
-      if (e < cnt) {
-        const uint32_t g = gauss[range.x + cstart + e];
-        sg[e] = g;
-        const float4 r0 = rec[4 * (size_t)g], r1 = rec[4 * (size_t)g + 1], r2 = rec[4 * (size_t)g + 2];
-        sxy[e] = make_float4(r0.x, r0.x, r0.y, r0.y);
-        sab[e] = make_float4(r0.z, r0.z, r0.w, r0.w);
-        sco[e] = make_float4(r1.x, r1.x, r1.y, r1.y);
-        srg[e] = make_float4(r1.w, r1.w, r2.x, r2.x);
-        sb[e] = make_float2(r2.y, r2.y);
-        ssig[e] = make_float2(r1.z, r1.z - kSigmaEdge);
-        srect[e] = tile_rect_masks<TW, TH>(fbits(r2.z), fbits(r2.w), ox, oy);
-        m = subblock_mask<TW, TH, SBH>(fbits(r2.z), fbits(r2.w), ox, oy);
-      }
-      smask[e] = (WarpMask)m;
+  // Entries at or past every pixel's n_contrib contribute nothing to the tile.
+  const uint32_t warp_last = __reduce_max_sync(0xffffffffu, max(last[0], last[1]));
+  if (lane == 0) atomicMax(&tile_last, warp_last);
+  wk.template barrier<Shape::kTiles>();
+  const uint32_t n = tile_last;
+  for (uint32_t first = 0; first < n; first += kListChunk) {
+    if (first) wk.template barrier<Shape::kTiles>();
+    const uint32_t total = min(n - first, (uint32_t)kListChunk);
+    wk.scan(list, n - 1u - first, -1, total);
+    wk.template barrier<Shape::kTiles>();
+    Stager<typename W::Mask> stager;
+    stager.start(&list, total, wk.sub, st.queue);
+    uint32_t g = 0, index = 0;
+    uint32_t m = stager.fetch(rec, st.s[0], kStage, &g, &index);
+    while (m) {
+    copy_async_wait();
+    __syncwarp();
+    if (lane < m) {
+      const float4 r0 = st.s[0][lane], r1 = st.s[1][lane], r2 = st.s[2][lane];
+      st.xy[lane] = make_float4(r0.x, r0.x, r0.y, r0.y);
+      st.ab[lane] = make_float4(r0.z, r0.z, r0.w, r0.w);
+      st.co[lane] = make_float4(r1.x, r1.x, r1.y, r1.z);
+      st.rg[lane] = make_float4(r1.w, r1.w, r2.x, r2.x);
+      st.bm[lane] = make_float4(r2.y, r2.y, bitsf(sub_block_mask(fbits(r2.z), fbits(r2.w), wk.bx, wk.by)),
+                                bitsf(n - 1u - first - index));
+      st.g[lane] = g;
     }
-    __syncthreads();
-    const uint32_t limit = warp_max_last > cstart ? warp_max_last - cstart : 0u;
-    const uint32_t nl = build_warp_list(smask, cnt, limit, list);
-    for (int i = (int)nl - 1; i >= 0; i--) {
-      const uint32_t kk = list[i];
-      const uint32_t k = cstart + kk;
-      const Mask rm = srect[kk];
-      const bool cov0 = (rm & bits0) == bits0 && k < last[0];
-      const bool cov1 = (rm & bits1) == bits1 && k < last[1];
+    __syncwarp();
+    const uint32_t cnt = m;
+    m = stager.fetch(rec, st.s[0], kStage, &g, &index);  // loads while this stage is walked
+    for (uint32_t j = 0; j < cnt; j++) {
+      const float4 exy = st.xy[j], eab = st.ab[j], eco = st.co[j], erg = st.rg[j], ebm = st.bm[j];
+      const uint32_t mask = fbits(ebm.z), place = fbits(ebm.w);
+      const bool cov0 = (mask & bits0) == bits0 && place < last[0];
+      const bool cov1 = (mask & bits1) == bits1 && place < last[1];
       if (kCount) npairs += (uint32_t)cov0 + (uint32_t)cov1;
-      const float4 exy = sxy[kk], eab = sab[kk], eco = sco[kk], erg = srg[kk];
-      const float2 eb = sb[kk], esig = ssig[kk];
-      const f2 mx = f2_make(exy.x, exy.y), my = f2_make(exy.z, exy.w);
-      const f2 A = f2_make(eab.x, eab.y), B = f2_make(eab.z, eab.w);
-      const f2 Cc = f2_make(eco.x, eco.y), op = f2_make(eco.z, eco.w);
-      const f2 dx = f2_sub(px, mx), dy = f2_sub(py, my);
+      const f2 dx = f2_sub(px, f2_make(exy.x, exy.y)), dy = f2_sub(py, f2_make(exy.z, exy.w));
       f2 adx, cdy, bdx;
-      const f2 sigma = paired_sigma(A, B, Cc, dx, dy, &adx, &cdy, &bdx);
       float s0, s1;
-      f2_split(sigma, s0, s1);
+      f2_split(paired_sigma(f2_make(eab.x, eab.y), f2_make(eab.z, eab.w), f2_make(eco.x, eco.y), dx, dy, &adx, &cdy,
+                            &bdx), s0, s1);
       // The reference's range test (false for NaN, as there), then the alpha test by sigma.
-      const bool in0 = cov0 && !(s0 < 0.0f) && !(s0 > esig.x);
-      const bool in1 = cov1 && !(s1 < 0.0f) && !(s1 > esig.x);
-      bool v0 = in0 && s0 <= esig.y, v1 = in1 && s1 <= esig.y;
+      const bool in0 = cov0 && !(s0 < 0.0f) && !(s0 > eco.w);
+      const bool in1 = cov1 && !(s1 < 0.0f) && !(s1 > eco.w);
+      const float sure = eco.w - kSigmaEdge;
+      bool v0 = in0 && s0 <= sure, v1 = in1 && s1 <= sure;
       const bool edge0 = in0 && !v0, edge1 = in1 && !v1;
       if (__any_sync(0xffffffffu, edge0 || edge1)) {  // rare: the correctly rounded exp decides
         if (edge0) v0 = !(eco.z * crm::expf_cr(-s0) < SPLAT_ALPHA_MIN);
-        if (edge1) v1 = !(eco.w * crm::expf_cr(-s1) < SPLAT_ALPHA_MIN);
+        if (edge1) v1 = !(eco.z * crm::expf_cr(-s1) < SPLAT_ALPHA_MIN);
       }
-      // No pixel of the warp takes the entry: every update below would be an identity.
-      if (!__any_sync(0xffffffffu, v0 || v1)) continue;
-      const float inf = __int_as_float(0x7f800000);
-      float g0, g1;
-      f2_split(f2_mul(f2_make(v0 ? s0 : inf, v1 ? s1 : inf), nlog2e), g0, g1);
-      f2 gv = f2_make(ex2_approx(g0), ex2_approx(g1));  // gauss (fast exp), 0 where skipped
-      f2 alpha = f2_mul(op, gv);
-      if (!(eco.z < SPLAT_ALPHA_MAX)) {
-        // Opacity >= 0.99 (uniform over the warp): alpha clamps at 0.99 and the gradients
-        // through sigma and opacity vanish there (rasterize.rs:414-432). Products within a
-        // relative band of the clamp are decided with the correctly rounded exp.
-        float a0, a1, q0, q1;
-        f2_split(alpha, a0, a1);
-        f2_split(gv, q0, q1);
-        if (fabsf(a0 - SPLAT_ALPHA_MAX) < SPLAT_ALPHA_MAX * kExpBand) {
-          q0 = crm::expf_cr(-s0);
-          a0 = eco.z * q0;
+      if (__any_sync(0xffffffffu, v0 || v1)) {  // else every update below would be an identity
+        const float inf = __int_as_float(0x7f800000);
+        float g0, g1;
+        f2_split(f2_mul(f2_make(v0 ? s0 : inf, v1 ? s1 : inf), nlog2e), g0, g1);
+        f2 gv = f2_make(ex2_approx(g0), ex2_approx(g1));  // gauss (fast exp), 0 where skipped
+        f2 alpha = f2_mul(f2_splat(eco.z), gv);
+        if (!(eco.z < SPLAT_ALPHA_MAX)) {
+          // Opacity >= 0.99 (uniform over the warp): alpha clamps at 0.99 and the gradients
+          // through sigma and opacity vanish there (rasterize.rs:414-432). Products within a
+          // relative band of the clamp are decided with the correctly rounded exp.
+          float a0, a1, q0, q1;
+          f2_split(alpha, a0, a1);
+          f2_split(gv, q0, q1);
+          if (fabsf(a0 - SPLAT_ALPHA_MAX) < SPLAT_ALPHA_MAX * kExpBand) {
+            q0 = crm::expf_cr(-s0);
+            a0 = eco.z * q0;
+          }
+          if (fabsf(a1 - SPLAT_ALPHA_MAX) < SPLAT_ALPHA_MAX * kExpBand) {
+            q1 = crm::expf_cr(-s1);
+            a1 = eco.z * q1;
+          }
+          gv = f2_make(a0 < SPLAT_ALPHA_MAX ? q0 : 0.0f, a1 < SPLAT_ALPHA_MAX ? q1 : 0.0f);
+          alpha = f2_make(fminf(a0, SPLAT_ALPHA_MAX), fminf(a1, SPLAT_ALPHA_MAX));
         }
-        if (fabsf(a1 - SPLAT_ALPHA_MAX) < SPLAT_ALPHA_MAX * kExpBand) {
-          q1 = crm::expf_cr(-s1);
-          a1 = eco.w * q1;
-        }
-        gv = f2_make(a0 < SPLAT_ALPHA_MAX ? q0 : 0.0f, a1 < SPLAT_ALPHA_MAX ? q1 : 0.0f);
-        alpha = f2_make(fminf(a0, SPLAT_ALPHA_MAX), fminf(a1, SPLAT_ALPHA_MAX));
+        // Values only from here on (fused, reciprocal for division).
+        float o0, o1;
+        f2_split(f2_sub(one, alpha), o0, o1);
+        const f2 inv = f2_make(rcp_fast(o0), rcp_fast(o1));
+        T = f2_mul(T, inv);
+        const f2 dr = f2_sub(f2_make(erg.x, erg.y), acc_r);
+        const f2 dg = f2_sub(f2_make(erg.z, erg.w), acc_g);
+        const f2 db = f2_sub(f2_make(ebm.x, ebm.y), acc_b);
+        f2 dalpha = f2_fma(db, d2, f2_fma(dg, d1, f2_mul(dr, d0)));
+        acc_r = f2_fma(alpha, dr, acc_r);
+        acc_g = f2_fma(alpha, dg, acc_g);
+        acc_b = f2_fma(alpha, db, acc_b);
+        dalpha = f2_fma(dalpha, T, f2_mul(nbg, inv));
+        float4 hw;
+        f2_split(f2_mul(gv, dalpha), hw.x, hw.y);
+        f2_split(f2_mul(alpha, T), hw.z, hw.w);
+        st.hw[count * kGroupRow + lane] = hw;
+        if ((lane & 7u) == count) mykk = j;
+        count++;
       }
-      // Values only from here on (fused, reciprocal for division).
-      float o0, o1;
-      f2_split(f2_sub(one, alpha), o0, o1);
-      const f2 inv = f2_make(rcp_fast(o0), rcp_fast(o1));
-      T = f2_mul(T, inv);
-      const f2 dr = f2_sub(f2_make(erg.x, erg.y), acc_r);
-      const f2 dg = f2_sub(f2_make(erg.z, erg.w), acc_g);
-      const f2 db = f2_sub(f2_make(eb.x, eb.y), acc_b);
-      f2 dalpha = f2_fma(db, d2, f2_fma(dg, d1, f2_mul(dr, d0)));
-      const f2 at = f2_mul(alpha, T);
-      acc_r = f2_fma(alpha, dr, acc_r);
-      acc_g = f2_fma(alpha, dg, acc_g);
-      acc_b = f2_fma(alpha, db, acc_b);
-      dalpha = f2_fma(dalpha, T, f2_mul(nbg, inv));
-      const f2 c5 = f2_mul(gv, dalpha);
-      // nds = opacity dalpha gauss = -dsigma; the signs are applied in the lane sums below.
-      const f2 nds = f2_mul(f2_mul(op, dalpha), gv);
-      const f2 ndx = f2_mul(nds, f2_fma(B, dy, adx));  // -ddx = -dsigma (A dx + B dy)
-      const f2 ndy = f2_mul(nds, f2_add(bdx, cdy));    // -ddy = -dsigma (B dx + C dy)
-      const f2 hs = f2_mul(half, nds);
-      const f2 c2 = f2_mul(f2_mul(hs, dx), dx);
-      const f2 c3 = f2_mul(f2_mul(nds, dx), dy);
-      const f2 c4 = f2_mul(f2_mul(hs, dy), dy);
-      const f2 c6 = f2_mul(at, d0), c7 = f2_mul(at, d1), c8 = f2_mul(at, d2);
-      float c[kSlots], lo, hi;
-      f2_split(ndx, lo, hi);
-      c[0] = lo + hi;
-      c[9] = fabsf(lo) + fabsf(hi);
-      f2_split(ndy, lo, hi);
-      c[1] = lo + hi;
-      c[10] = fabsf(lo) + fabsf(hi);
-      f2_split(c2, lo, hi);
-      c[2] = -lo - hi;
-      f2_split(c3, lo, hi);
-      c[3] = -lo - hi;
-      f2_split(c4, lo, hi);
-      c[4] = -lo - hi;
-      f2_split(c5, lo, hi);
-      c[5] = lo + hi;
-      f2_split(c6, lo, hi);
-      c[6] = lo + hi;
-      f2_split(c7, lo, hi);
-      c[7] = lo + hi;
-      f2_split(c8, lo, hi);
-      c[8] = lo + hi;
-      f2_split(at, lo, hi);
-      c[11] = lo + hi;
-      const float tot = warp_transpose_reduce12(c);
-      const uint32_t local = (lane >> 1) & 3u;
-      const uint32_t slot = 6u * ((lane >> 4) & 1u) + 3u * ((lane >> 3) & 1u) + local;
-      if (!(lane & 1u) && local < 3u) atomicAdd(&acc[kk * kSlots + slot], tot);
+      if (count == kGroup || (j + 1u == cnt && count)) {
+        __syncwarp();
+        reduce_group(st, count, mykk, px0, py0, pgrad, cap);
+        count = 0;
+      }
     }
-    __syncthreads();
-#pragma unroll
-    for (uint32_t e = threadIdx.x; e < (uint32_t)CH; e += NT) {
-      if (e >= cnt) break;
-      float* a = &acc[e * kSlots];
-      const size_t g = sg[e];
-      const float4 v0 = make_float4(a[0], a[1], a[2], a[3]);
-      const float4 v1 = make_float4(a[4], a[5], a[6], a[7]);
-      const float4 v2 = make_float4(a[8], a[9], a[10], a[11]);
-      if (v0.x != 0.0f || v0.y != 0.0f || v0.z != 0.0f || v0.w != 0.0f) atomicAdd(&pgrad[g], v0);
-      if (v1.x != 0.0f || v1.y != 0.0f || v1.z != 0.0f || v1.w != 0.0f) atomicAdd(&pgrad[cap + g], v1);
-      if (v2.x != 0.0f || v2.y != 0.0f || v2.z != 0.0f || v2.w != 0.0f) atomicAdd(&pgrad[2 * cap + g], v2);
-#pragma unroll
-      for (int q = 0; q < kSlots; q++) a[q] = 0.0f;
     }
-    __syncthreads();
-    cend = cstart;
   }
   if (kCount) {
     unsigned long long np = npairs;
@@ -1177,45 +1433,51 @@ Status launch_raster_bwd_det(Ctx* c, const float* proj, const uint32_t* gauss, c
     else return Status::make(SPLAT_ERR_INVALID, "unsupported raster configuration");           \
   } while (0)
 
-constexpr int kFwdChunk = 256;
+// Launches a walking kernel over `tiles` tiles. Its shared memory is above the default limit,
+// which is raised on the kernel's first use on a device.
+template <typename Shape, typename Smem, typename... P, typename... A>
+static Status launch_walk(Ctx* c, void (*kernel)(P...), uint32_t tiles, A... args) {
+  static std::mutex guard;
+  static std::set<std::pair<int, const void*>> ready;
+  {
+    std::lock_guard<std::mutex> lock(guard);
+    const std::pair<int, const void*> key(c->device, reinterpret_cast<const void*>(kernel));
+    if (!ready.count(key)) {
+      SPLAT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem)));
+      ready.insert(key);
+    }
+  }
+  kernel<<<ceil_div(tiles, Shape::kTiles), 32 * Shape::kWarps, sizeof(Smem), c->stream>>>(args...);
+  c->launches.count++;
+  SPLAT_LAUNCHED("compositing kernel");
+  return Status::ok();
+}
 
 Status launch_raster_fwd(Ctx* c, const float* proj, const uint32_t* gauss, const uint32_t* ranges, uint32_t width,
                          uint32_t height, const float bg[3], float* image, float* final_t, uint32_t* n_contrib,
                          uint64_t* pairs, const BatchTable* bt, uint32_t tiles_cap) {
   const RasterConfig& rc = c->raster;
   const uint32_t tiles_x = rc.tiles_x(width);
-  const uint32_t blocks = bt ? tiles_cap : rc.tiles(width, height);
-  if (blocks == 0) return Status::ok();
-// With the 16-column tiles the forward stages chunks of kFwdChunk entries whatever the
-// configuration's chunk depth (which then sets the backward's): fewer chunks mean fewer block
-// barriers, and 256 was the faster forward on both shapes (16x16: 0.553 ms against 0.570
-// with 128; 16x32: 0.585 against 0.616). 8x8 tiles (two warps) keep the configured depth.
-#define SPLAT_FWD(TW, TH, CH, K)                                                                                  \
-  raster_fwd_kernel<TW, TH, CH, K><<<blocks, TW * TH, 0, c->stream>>>(                                           \
-      reinterpret_cast<const float4*>(proj), gauss, reinterpret_cast<const uint2*>(ranges), width, height, tiles_x, \
-      bg[0], bg[1], bg[2], image, final_t, n_contrib, reinterpret_cast<unsigned long long*>(pairs), bt)
-#define SPLAT_FWD8(TW, TH, CH) \
-  if (pairs) SPLAT_FWD(TW, TH, CH, true); else SPLAT_FWD(TW, TH, CH, false)
-  const bool count = pairs != nullptr;
+  const uint32_t tiles = bt ? tiles_cap : rc.tiles(width, height);
+  if (tiles == 0) return Status::ok();
+#define SPLAT_FWDK(TW, TH, K)                                                                                     \
+  SPLAT_TRY((launch_walk<FwdShape<TW, TH>, FwdSmem<TW, TH>>(                                                     \
+      c, raster_fwd_kernel<TW, TH, K>, tiles, reinterpret_cast<const float4*>(proj), gauss,                      \
+      reinterpret_cast<const uint2*>(ranges), tiles, width, height, tiles_x, bg[0], bg[1], bg[2], image, final_t, \
+      n_contrib, reinterpret_cast<unsigned long long*>(pairs), bt)))
+#define SPLAT_FWD(TW, TH) \
+  if (pairs) SPLAT_FWDK(TW, TH, true); else SPLAT_FWDK(TW, TH, false)
   if (rc.tile_w == 16 && rc.tile_h == 16) {
-    if (count) SPLAT_FWD(16, 16, kFwdChunk, true); else SPLAT_FWD(16, 16, kFwdChunk, false);
+    SPLAT_FWD(16, 16);
   } else if (rc.tile_w == 16 && rc.tile_h == 32) {
-    if (count) SPLAT_FWD(16, 32, kFwdChunk, true); else SPLAT_FWD(16, 32, kFwdChunk, false);
-  } else if (rc.tile_w == 8 && rc.tile_h == 8 && rc.chunk == 256) {
-    SPLAT_FWD8(8, 8, 256);
-  } else if (rc.tile_w == 8 && rc.tile_h == 8 && rc.chunk == 128) {
-    SPLAT_FWD8(8, 8, 128);
-  } else if (rc.tile_w == 8 && rc.tile_h == 8 && rc.chunk == 64) {
-    SPLAT_FWD8(8, 8, 64);
-  } else if (rc.tile_w == 8 && rc.tile_h == 8 && rc.chunk == 32) {
-    SPLAT_FWD8(8, 8, 32);
+    SPLAT_FWD(16, 32);
+  } else if (rc.tile_w == 8 && rc.tile_h == 8) {
+    SPLAT_FWD(8, 8);
   } else {
     return Status::make(SPLAT_ERR_INVALID, "unsupported raster configuration");
   }
-#undef SPLAT_FWD8
 #undef SPLAT_FWD
-  c->launches.count++;
-  SPLAT_LAUNCHED("raster_fwd_kernel");
+#undef SPLAT_FWDK
   return Status::ok();
 }
 
@@ -1233,20 +1495,26 @@ Status launch_raster_bwd(Ctx* c, const float* proj, const uint32_t* gauss, const
       bg[0], bg[1], bg[2], final_t, n_contrib, dimage, reinterpret_cast<float4*>(pgrad), cap,                     \
       reinterpret_cast<unsigned long long*>(pairs), bt)
 #define SPLAT_BWD1(TW, TH, CH) SPLAT_BWD(TW, TH, CH, 1)
-#define SPLAT_BWD2X(TW, TH, CH, K)                                                                                \
-  raster_bwd_x2_kernel<TW, TH, CH, K><<<blocks, TW * TH / 2, 0, c->stream>>>(                                    \
-      reinterpret_cast<const float4*>(proj), gauss, reinterpret_cast<const uint2*>(ranges), width, height, tiles_x, \
-      bg[0], bg[1], bg[2], final_t, n_contrib, dimage, reinterpret_cast<float4*>(pgrad), cap,                     \
-      reinterpret_cast<unsigned long long*>(pairs), bt)
-#define SPLAT_BWD2(TW, TH, CH) SPLAT_BWD2X(TW, TH, CH, false)
-#define SPLAT_BWD2C(TW, TH, CH) SPLAT_BWD2X(TW, TH, CH, true)
-  if (rc.ppl == 2 && pairs)
-    SPLAT_RASTER_DISPATCH(rc, SPLAT_BWD2C);
-  else if (rc.ppl == 2)
-    SPLAT_RASTER_DISPATCH(rc, SPLAT_BWD2);
-  else
-    SPLAT_RASTER_DISPATCH(rc, SPLAT_BWD1);
-#undef SPLAT_BWD2C
+#define SPLAT_BWD2X(TW, TH, K)                                                                                    \
+  SPLAT_TRY((launch_walk<BwdShape<TW, TH>, BwdSmem<TW, TH>>(                                                     \
+      c, raster_bwd_x2_kernel<TW, TH, K>, blocks, reinterpret_cast<const float4*>(proj), gauss,                  \
+      reinterpret_cast<const uint2*>(ranges), blocks, width, height, tiles_x, bg[0], bg[1], bg[2], final_t,      \
+      n_contrib, dimage, reinterpret_cast<float4*>(pgrad), cap, reinterpret_cast<unsigned long long*>(pairs), bt)))
+#define SPLAT_BWD2(TW, TH) \
+  if (pairs) SPLAT_BWD2X(TW, TH, true); else SPLAT_BWD2X(TW, TH, false)
+  if (rc.ppl == 2) {
+    if (rc.tile_w == 16 && rc.tile_h == 16) {
+      SPLAT_BWD2(16, 16);
+    } else if (rc.tile_w == 16 && rc.tile_h == 32) {
+      SPLAT_BWD2(16, 32);
+    } else if (rc.tile_w == 8 && rc.tile_h == 8) {
+      SPLAT_BWD2(8, 8);
+    } else {
+      return Status::make(SPLAT_ERR_INVALID, "unsupported raster configuration");
+    }
+    return Status::ok();
+  }
+  SPLAT_RASTER_DISPATCH(rc, SPLAT_BWD1);
 #undef SPLAT_BWD2
 #undef SPLAT_BWD2X
 #undef SPLAT_BWD1
