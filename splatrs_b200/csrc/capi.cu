@@ -309,9 +309,11 @@ SPLAT_API int splat_bin_count(splat_ctx* ctx, const uint32_t* num_tiles_dev, int
   Enter e(ctx);
   uint64_t* total = nullptr;
   Status s = arena_reserve(&ctx->c, 8, (void**)&total);
-  if (s.good()) s = launch_scan_u32(&ctx->c, num_tiles_dev, n, entry_offset_dev, 1, total);
-  uint64_t* h = reinterpret_cast<uint64_t*>(ctx->c.host_small);
-  if (s.good()) s = cuda_status(cudaMemcpyAsync(h, total, 8, cudaMemcpyDeviceToHost, ctx->c.stream), "read entry count");
+  // The scan stores the count into mapped host memory: the read-back is no copy of its own.
+  if (s.good())
+    s = launch_scan_u32(&ctx->c, num_tiles_dev, n, entry_offset_dev, 1, total,
+                        static_cast<uint64_t*>(ctx->c.host_small_dev));
+  const volatile uint64_t* h = static_cast<const volatile uint64_t*>(ctx->c.host_small);
   if (s.good()) s = cuda_status(cudaStreamSynchronize(ctx->c.stream), "cudaStreamSynchronize");
   if (s.good()) s = take_sort_error(&ctx->c);
   if (!s.good()) return fail(ctx, s);
@@ -330,8 +332,8 @@ SPLAT_API int splat_bin_sort(splat_ctx* ctx, const float* proj_dev, const uint32
       (num_entries && (!proj_dev || !entry_offset_dev || !gauss_dev)))
     return invalid(ctx, "splat_bin_sort: bad buffers");
   Enter e(ctx);
-  uint32_t* h = reinterpret_cast<uint32_t*>(ctx->c.host_small);
-  Status s = cuda_status(cudaMemcpyAsync(h, depth_range_dev, 8, cudaMemcpyDeviceToHost, ctx->c.stream), "read depth range");
+  const volatile uint32_t* h = static_cast<const volatile uint32_t*>(ctx->c.host_small);
+  Status s = launch_publish_u32(&ctx->c, depth_range_dev, 2, nullptr, 0);
   if (s.good()) s = cuda_status(cudaStreamSynchronize(ctx->c.stream), "cudaStreamSynchronize");
   if (s.good()) s = take_sort_error(&ctx->c);  // of an earlier sort on this context
   if (!s.good()) return fail(ctx, s);

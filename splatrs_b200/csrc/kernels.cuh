@@ -82,7 +82,12 @@ Status launch_project_bwd_batch_adam(Ctx* c, float* planes, float* m, float* v, 
 // gradient at the copy's values, updates the f32 master and rewrites the copy.
 Status launch_planes_to_bf16(Ctx* c, const float* planes, int64_t n, int64_t cap, void* bf16);
 
-Status launch_scan_u32(Ctx* c, const uint32_t* in, int64_t n, uint32_t* out, int write_total, uint64_t* total_dev);
+// Exclusive scan; the total goes to *total_dev, out[n] (write_total) and *host_total (the device
+// alias of mapped host memory; may be NULL).
+Status launch_scan_u32(Ctx* c, const uint32_t* in, int64_t n, uint32_t* out, int write_total, uint64_t* total_dev,
+                       uint64_t* host_total = nullptr);
+// (smallest, largest) depth bits to (0xffffffff, 0).
+Status launch_reset_range(Ctx* c, uint32_t* range);
 
 // Binning without a host read-back: the entry count (*E_dev, from the entry-offset scan)
 // and the depth range stay on the device; `scratch` holds dev_sort_scratch_bytes(E_cap)
@@ -158,7 +163,7 @@ Status launch_publish_u32(Ctx* c, const uint32_t* a, int na, const uint32_t* b, 
 // The same into another mapped host buffer (its device alias `out_dev`).
 Status launch_publish_u32_to(Ctx* c, const uint32_t* a, int na, const uint32_t* b, int nb, void* out_dev);
 Status launch_scan_u32_into(Ctx* c, const uint32_t* in, int64_t n, uint32_t* out, int write_total,
-                            uint64_t* partial, uint64_t* total);
+                            uint64_t* partial, uint64_t* total, uint64_t* host_total = nullptr);
 constexpr int kScanValuesPerBlock = 4096;
 Status launch_bin_sort(Ctx* c, const float* proj, const uint32_t* entry_offset, int64_t n, int64_t E,
                        const uint32_t* depth_range_dev, uint32_t depth_min, uint32_t depth_max, uint32_t width,
