@@ -204,6 +204,8 @@ Status launch_diag_pair_exact(Ctx* c, uint32_t n, uint32_t* out_host);
 // Throughput of one unit (0: FP32 FMA, in FLOP/s; 1: MUFU ex2, in operations/s), peaks.cu.
 Status launch_diag_peak(Ctx* c, int unit, double* ops_per_s, float* ms_out);
 
+// Edge of a loss block's tile in a batch's table (BatchTable::loss_start).
+constexpr int kLossTile = 32;
 Status launch_loss(Ctx* c, const float* pred, const void* target, int target_u8, uint32_t width, uint32_t height,
                    float lambda, float* grad, float* out3, const StepParams* sp = nullptr,
                    const BatchTable* bt = nullptr, uint32_t blocks_cap = 0, uint64_t pix_cap = 0);

@@ -430,7 +430,7 @@ void fill_batch_table(splat_trainer* t, const IterPlan& p, BatchTable& b) {
     const View& v = *t->views[p.views[k]];
     const splat_camera& vc = plan_cam(p, v);
     const uint32_t tx = t->c->raster.tiles_x(vc.width), ty = t->c->raster.tiles_y(vc.height);
-    const uint32_t lx = (vc.width + 31) / 32, ly = (vc.height + 31) / 32;
+    const uint32_t lx = ceil_div(vc.width, kLossTile), ly = ceil_div(vc.height, kLossTile);
     b.cam[k] = vc;
     b.target[k] = plan_rgb(p, v);
     b.tiles_x[k] = tx;
@@ -465,7 +465,7 @@ void size_batch_caps(splat_trainer* t) {
   for (const View* v : t->views) {
     const uint32_t w = v->cam.width, h = v->cam.height;
     most_tiles = std::max(most_tiles, t->c->raster.tiles(w, h));
-    most_loss = std::max(most_loss, ((w + 31) / 32) * ((h + 31) / 32));
+    most_loss = std::max(most_loss, ceil_div(w, kLossTile) * ceil_div(h, kLossTile));
     most_pix = std::max<uint64_t>(most_pix, (uint64_t)w * h);
   }
   t->tiles_cap = most_tiles * t->batch;
