@@ -788,6 +788,42 @@ __device__ __forceinline__ void proj_grad_one(const GParams& g, const splat_came
   }
 }
 
+// Adam's operands of a thread's Gaussian (parameters, first and second moments, plane by plane)
+// on their way through shared memory: kAhead planes are in flight as asynchronous copies while
+// the gradients are computed and while earlier planes are updated. Every thread copies and reads
+// its own Gaussian's values, so a thread waits for its own copies and for nobody else. Without
+// this each plane's three loads started after the previous plane's stores: 24 KB in flight per
+// SM, a third of the memory's rate.
+template <int NT, int kAhead>
+struct AdamStage {
+  float4 p[kAhead][NT], m[kAhead][NT], v[kAhead][NT];
+};
+__device__ __forceinline__ void copy_async16(float4* smem, const float4* global) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(global) : "memory");
+}
+template <int NT, int kAhead>
+__device__ __forceinline__ void adam_prefetch(AdamStage<NT, kAhead>& st, int q, const float4* p, const float4* m,
+                                              const float4* v, int64_t cap, int64_t i) {
+  if (q < kPlanes) {
+    const int64_t o = (int64_t)q * cap + i;
+    const int s = q % kAhead, t = threadIdx.x;
+    copy_async16(&st.p[s][t], p + o);
+    copy_async16(&st.m[s][t], m + o);
+    copy_async16(&st.v[s][t], v + o);
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");  // one group per plane, empty past the last
+}
+// Plane q's operands, once its group has landed (the kAhead - 1 younger ones may still fly).
+template <int NT, int kAhead>
+__device__ __forceinline__ void adam_take(const AdamStage<NT, kAhead>& st, int q, float4& p, float4& m, float4& v) {
+  asm volatile("cp.async.wait_group %0;" ::"n"(kAhead - 1) : "memory");
+  const int s = q % kAhead, t = threadIdx.x;
+  p = st.p[s][t];
+  m = st.m[s][t];
+  v = st.v[s][t];
+}
+
 // project_backward_one (project.rs:335-474), plus DensifyStats::accumulate
 // (densify.rs:36-60) when `stats` is given. With ADAM the 59 gradients never leave the
 // registers: Adam::step (adam.rs:77-161) updates the parameters in place and the moments m
@@ -797,6 +833,7 @@ __device__ __forceinline__ void proj_grad_one(const GParams& g, const splat_came
 // HBM-bound kernel); capped at 128 the kernel spills a few hundred bytes to L1 and runs
 // 22-23% faster (measured at 1M Gaussians: 0.606 -> 0.475 ms with Adam, 0.149 -> 0.115 ms
 // without).
+constexpr int kAdamAhead = 5;
 template <int DEG, bool ADAM, bool BF16>
 __global__ void __launch_bounds__(128, 4) project_bwd_kernel(const float4* __restrict__ planes, int64_t n, int64_t cap,
                                                           splat_camera cam_arg, splat_proj_opts opts,
@@ -812,6 +849,11 @@ __global__ void __launch_bounds__(128, 4) project_bwd_kernel(const float4* __res
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   if (ADAM && skip && *skip) return;
+  __shared__ AdamStage<128, ADAM ? kAdamAhead : 1> st;
+  if (ADAM) {
+#pragma unroll
+    for (int q = 0; q < kAdamAhead; q++) adam_prefetch(st, q, planes, adam_m, adam_v, cap, i);
+  }
   const splat_camera cam = sp ? sp->cam : cam_arg;
   const AdamArgs adam = (ADAM && sp) ? sp->adam : adam_arg;
   const float4 g0 = pgrad[i], g1 = pgrad[cap + i], g2 = pgrad[2 * cap + i];
@@ -865,11 +907,13 @@ __global__ void __launch_bounds__(128, 4) project_bwd_kernel(const float4* __res
       else
         g = make_float4(o_sh[4 * (q - 3)], o_sh[4 * (q - 3) + 1], o_sh[4 * (q - 3) + 2], o_sh[4 * (q - 3) + 3]);
       const int64_t o = (int64_t)q * cap + i;
-      float4 p = pw[o], m = adam_m[o], v = adam_v[o];
+      float4 p, m, v;
+      adam_take(st, q, p, m, v);
       adam_plane(adam, q, p, g, m, v);
       pw[o] = p;
       adam_m[o] = m;
       adam_v[o] = v;
+      adam_prefetch(st, q + kAdamAhead, pw, adam_m, adam_v, cap, i);
       // The render copy follows the f32 master (round to nearest even).
       if (BF16 && q > 0) bf[(int64_t)(q - 1) * cap + i] = pack_bf16x4(p);
     }
@@ -1055,6 +1099,7 @@ Status launch_project_bwd_adam(Ctx* c, float* planes, float* m, float* v, int64_
 // in view order, into a per-thread column of shared memory together with the view's
 // densification statistics; Adam then updates the parameters once with the sum.
 constexpr int kBatchBwdThreads = 128;
+constexpr int kBatchAhead = 2;  // what fits beside the gradient columns in 48 KB
 
 template <int DEG, bool BF16>
 __global__ void __launch_bounds__(kBatchBwdThreads) project_bwd_batch_adam_kernel(
@@ -1067,6 +1112,9 @@ __global__ void __launch_bounds__(kBatchBwdThreads) project_bwd_batch_adam_kerne
   if (i >= n) return;
   if (skip && *skip) return;
   const int tid = threadIdx.x;
+  __shared__ AdamStage<kBatchBwdThreads, kBatchAhead> st;
+#pragma unroll
+  for (int q = 0; q < kBatchAhead; q++) adam_prefetch(st, q, planes, adam_m, adam_v, cap, i);
 #pragma unroll
   for (int f = 0; f < kPlanes * 4; f++) acc[f][tid] = 0.0f;
   GParams g;
@@ -1110,11 +1158,13 @@ __global__ void __launch_bounds__(kBatchBwdThreads) project_bwd_batch_adam_kerne
   for (int q = 0; q < kPlanes; q++) {
     const float4 gq = make_float4(acc[4 * q][tid], acc[4 * q + 1][tid], acc[4 * q + 2][tid], acc[4 * q + 3][tid]);
     const int64_t o = (int64_t)q * cap + i;
-    float4 p = planes[o], m = adam_m[o], v = adam_v[o];
+    float4 p, m, v;
+    adam_take(st, q, p, m, v);
     adam_plane(adam, q, p, gq, m, v);
     planes[o] = p;
     adam_m[o] = m;
     adam_v[o] = v;
+    adam_prefetch(st, q + kBatchAhead, planes, adam_m, adam_v, cap, i);
     if (BF16 && q > 0) bf[(int64_t)(q - 1) * cap + i] = pack_bf16x4(p);
   }
 }
