@@ -72,7 +72,11 @@ __device__ __forceinline__ void finalize_loss(const double* __restrict__ partial
 }
 
 // ---------------------------------------------------------------------------------------
-// Large views: a block takes all channels of a 32 x 32 tile in turn, two outputs per thread.
+// Large views: a block takes all channels of a 32 x 32 tile in turn, two outputs per thread. The
+// blocks' sums go to slots that the backward's first block adds up (no launch to clear, no launch
+// to finish): 1297x840 120 -> 108 us, 1920x1080 206 -> 192 us for the whole loss. Tiles of 64 rows
+// with eight outputs per thread and one channel per block were slower here (121 and 248 us: every
+// channel's block reads the interleaved pixels again).
 // ---------------------------------------------------------------------------------------
 constexpr int kLT = kLossTile;     // output tile edge
 constexpr int kLE = kLT + 2 * kHalo;
@@ -689,6 +693,9 @@ constexpr int kSmallTileH = 16;
 Status launch_loss(Ctx* c, const float* pred, const void* target, int target_u8, uint32_t width, uint32_t height,
                    float lambda, float* grad, float* out3, const StepParams* sp, const BatchTable* bt,
                    uint32_t blocks_cap, uint64_t pix_cap) {
+  // The line between the two: 32 x 32 tiles per SM. Below 4 the small kernels (640x480 39 us against
+  // 58, 800x600 53 against 69); at 1297x840 (7.4) they are even (109 and 108 us) and at 1920x1080
+  // (13.8) the large ones lead (192 against 211). A batch's table counts 32 x 32 tiles.
   const uint64_t tiles = (uint64_t)ceil_div(width, kLT) * ceil_div(height, kLT);
   const bool small = !bt && tiles < 4 * (uint64_t)c->sm_count;
   const dim3 grid = bt      ? dim3(blocks_cap)
