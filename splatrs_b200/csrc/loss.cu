@@ -91,6 +91,7 @@ __global__ void __launch_bounds__(kLossThreads) ssim_fwd_kernel(const float* __r
                                                                 float* __restrict__ dmaps, double* __restrict__ sums,
                                                                 const StepParams* __restrict__ sp,
                                                                 const BatchTable* __restrict__ bt) {
+  chain_begin();
   const void* target = sp ? sp->target : target_arg;
   int bxi = blockIdx.x, byi = blockIdx.y;
   if (bt) {  // a batch: flat block index -> view, block within the view, buffer offsets
@@ -259,6 +260,7 @@ __global__ void __launch_bounds__(kLossThreads) ssim_bwd_kernel(const float* __r
                                                                 float* __restrict__ grad, float* __restrict__ out3,
                                                                 const StepParams* __restrict__ sp,
                                                                 const BatchTable* __restrict__ bt) {
+  chain_begin();
   __shared__ double red[3][kLossThreads / 32];
   if (blockIdx.x == 0 && blockIdx.y == 0) {
     if (bt) {
@@ -458,6 +460,7 @@ __global__ void __launch_bounds__(SmallShape<TH>::kThreads) ssim_fwd_small_kerne
     const float* __restrict__ pred, const void* __restrict__ target_arg, int target_u8, uint32_t width_arg,
     uint32_t height_arg, LossKernel K, float* __restrict__ dmaps, double* __restrict__ partial,
     const StepParams* __restrict__ sp) {
+  chain_begin();
   typedef SmallShape<TH> S;
   extern __shared__ __align__(16) unsigned char loss_smem[];
   FwdTile<TH>& t = *reinterpret_cast<FwdTile<TH>*>(loss_smem);
@@ -586,6 +589,7 @@ __global__ void __launch_bounds__(SmallShape<TH>::kThreads) ssim_bwd_small_kerne
     const float* __restrict__ pred, const void* __restrict__ target_arg, int target_u8, uint32_t width_arg,
     uint32_t height_arg, LossKernel K, const float* __restrict__ dmaps, const double* __restrict__ partial,
     float lambda, float* __restrict__ grad, float* __restrict__ out3, const StepParams* __restrict__ sp) {
+  chain_begin();
   typedef SmallShape<TH> S;
   extern __shared__ __align__(16) unsigned char loss_smem[];
   BwdTile<TH>& t = *reinterpret_cast<BwdTile<TH>*>(loss_smem);
@@ -709,18 +713,18 @@ Status launch_loss(Ctx* c, const float* pred, const void* target, int target_u8,
   if (small) {
     typedef SmallShape<kSmallTileH> S;
     static_assert(sizeof(FwdTile<kSmallTileH>) <= 48 * 1024 && sizeof(BwdTile<kSmallTileH>) <= 48 * 1024, "");
-    ssim_fwd_small_kernel<kSmallTileH><<<grid, S::kThreads, sizeof(FwdTile<kSmallTileH>), c->stream>>>(
-        pred, target, target_u8, width, height, K, dmaps, sums, sp);
-    ssim_bwd_small_kernel<kSmallTileH><<<grid, S::kThreads, sizeof(BwdTile<kSmallTileH>), c->stream>>>(
-        pred, target, target_u8, width, height, K, dmaps, sums, lambda, grad, out3, sp);
+    SPLAT_TRY(launch_chained(c, "ssim_fwd_small_kernel", ssim_fwd_small_kernel<kSmallTileH>, grid, S::kThreads,
+                             sizeof(FwdTile<kSmallTileH>), pred, target, target_u8, width, height, K, dmaps, sums,
+                             sp));
+    SPLAT_TRY(launch_chained(c, "ssim_bwd_small_kernel", ssim_bwd_small_kernel<kSmallTileH>, grid, S::kThreads,
+                             sizeof(BwdTile<kSmallTileH>), pred, target, target_u8, width, height, K, dmaps, sums,
+                             lambda, grad, out3, sp));
   } else {
-    ssim_fwd_kernel<<<grid, kLossThreads, 0, c->stream>>>(pred, target, target_u8, width, height, K, dmaps, sums, sp,
-                                                          bt);
-    ssim_bwd_kernel<<<grid, kLossThreads, 0, c->stream>>>(pred, target, target_u8, width, height, K, dmaps, sums,
-                                                          lambda, grad, out3, sp, bt);
+    SPLAT_TRY(launch_chained(c, "ssim_fwd_kernel", ssim_fwd_kernel, grid, kLossThreads, 0, pred, target, target_u8,
+                             width, height, K, dmaps, sums, sp, bt));
+    SPLAT_TRY(launch_chained(c, "ssim_bwd_kernel", ssim_bwd_kernel, grid, kLossThreads, 0, pred, target, target_u8,
+                             width, height, K, dmaps, sums, lambda, grad, out3, sp, bt));
   }
-  c->launches.count += 2;
-  SPLAT_LAUNCHED("loss kernels");
   return Status::ok();
 }
 

@@ -518,6 +518,7 @@ __global__ void __launch_bounds__(256) project_fwd_kernel(const float4* __restri
                                                           const uint2* __restrict__ bf,
                                                           const BatchTable* __restrict__ bt, uint32_t tile_w,
                                                           uint32_t tile_h) {
+  chain_begin();
   // A batch launch has one grid row per view; its records follow view-major.
   const int view = bt ? (int)blockIdx.y : 0;
   if (bt && view >= bt->views) return;
@@ -564,6 +565,7 @@ __global__ void __launch_bounds__(256) project_fwd_kernel(const float4* __restri
 __global__ void proj_from_reference_kernel(const float* __restrict__ p15, int64_t n, uint32_t width, uint32_t height,
                                            float4* __restrict__ rec, uint32_t* __restrict__ num_tiles,
                                            uint32_t* __restrict__ depth_range, uint32_t tile_w, uint32_t tile_h) {
+  chain_begin();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   bool visible = false;
   float depth = 0.0f;
@@ -847,6 +849,7 @@ __global__ void __launch_bounds__(128, 4) project_bwd_kernel(const float4* __res
                                                           AdamArgs adam_arg, const uint32_t* __restrict__ skip,
                                                           const StepParams* __restrict__ sp, uint2* bf,
                                                           float* __restrict__ stat_maxg) {
+  chain_begin();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   if (ADAM && skip && *skip) return;
@@ -958,6 +961,7 @@ __global__ void __launch_bounds__(kConvG) aos_to_planes_kernel(const float* __re
 
 __global__ void __launch_bounds__(kConvG) planes_to_aos_kernel(const float4* __restrict__ planes, int64_t n, int64_t cap,
                                                                float* __restrict__ aos) {
+  chain_begin();
   __shared__ float tile[kConvG][61];
   const int64_t base = (int64_t)blockIdx.x * kConvG;
   const int cnt = (int)min((int64_t)kConvG, n - base);
@@ -994,9 +998,9 @@ Status launch_project_fwd(Ctx* c, const float* planes, int64_t n, int64_t cap, c
   float4* r = reinterpret_cast<float4*>(proj);
   const uint2* bf = static_cast<const uint2*>(bf16);
 #define SPLAT_PFWD(D, B) \
-  project_fwd_kernel<D, B><<<dim3(grid, bt ? kMaxViews : 1), bs, 0, c->stream>>>(p, n, cap, cam, opts, r, num_tiles, \
+  SPLAT_TRY(launch_chained(c, "project_fwd_kernel", project_fwd_kernel<D, B>, dim3(grid, bt ? kMaxViews : 1), bs, 0, p, n, cap, cam, opts, r, num_tiles, \
                                                                                  depth_range, sp, bf, bt, \
-                                                                                 c->raster.tile_w, c->raster.tile_h)
+                                                                                 c->raster.tile_w, c->raster.tile_h))
   if (bf) {
     switch (opts.sh_degree) {
       case 0: SPLAT_PFWD(0, true); break;
@@ -1013,8 +1017,6 @@ Status launch_project_fwd(Ctx* c, const float* planes, int64_t n, int64_t cap, c
     }
   }
 #undef SPLAT_PFWD
-  c->launches.count++;
-  SPLAT_LAUNCHED("project_fwd_kernel");
   return Status::ok();
 }
 
@@ -1022,12 +1024,9 @@ Status launch_proj_from_reference(Ctx* c, const float* p15, int64_t n, uint32_t 
                                   uint32_t* num_tiles, uint32_t* depth_range) {
   SPLAT_TRY(launch_reset_range(c, depth_range));
   if (n == 0) return Status::ok();
-  proj_from_reference_kernel<<<ceil_div(n, 256), 256, 0, c->stream>>>(p15, n, width, height,
-                                                                       reinterpret_cast<float4*>(proj), num_tiles,
-                                                                       depth_range, c->raster.tile_w,
-                                                                       c->raster.tile_h);
-  c->launches.count++;
-  SPLAT_LAUNCHED("proj_from_reference_kernel");
+  SPLAT_TRY(launch_chained(c, "proj_from_reference_kernel", proj_from_reference_kernel, ceil_div(n, 256), 256, 0,
+                           p15, n, width, height, reinterpret_cast<float4*>(proj), num_tiles, depth_range,
+                           c->raster.tile_w, c->raster.tile_h));
   return Status::ok();
 }
 
@@ -1063,7 +1062,8 @@ static Status project_bwd_launch(Ctx* c, const float* planes, int64_t n, int64_t
     if (with_maxg) smg = reinterpret_cast<float*>(sm + cap);
   }
 #define SPLAT_PBWD(D) \
-  project_bwd_kernel<D, ADAM, BF16><<<grid, bs, 0, c->stream>>>(p, n, cap, cam, opts, r, pg, o, sa, sd, sm, absgrad, am, av, adam, skip, sp, bf, smg)
+  SPLAT_TRY(launch_chained(c, "project_bwd_kernel", project_bwd_kernel<D, ADAM, BF16>, grid, bs, 0, p, n, cap, cam,
+                           opts, r, pg, o, sa, sd, sm, absgrad, am, av, adam, skip, sp, bf, smg))
   switch (opts.sh_degree) {
     case 0: SPLAT_PBWD(0); break;
     case 1: SPLAT_PBWD(1); break;
@@ -1071,8 +1071,6 @@ static Status project_bwd_launch(Ctx* c, const float* planes, int64_t n, int64_t
     default: SPLAT_PBWD(3); break;
   }
 #undef SPLAT_PBWD
-  c->launches.count++;
-  SPLAT_LAUNCHED("project_bwd_kernel");
   return Status::ok();
 }
 
@@ -1108,6 +1106,7 @@ __global__ void __launch_bounds__(kBatchBwdThreads) project_bwd_batch_adam_kerne
     const float4* __restrict__ pgrad, int64_t pcap, float* __restrict__ stat_accum, uint32_t* __restrict__ stat_denom,
     uint32_t* __restrict__ stat_maxr, int absgrad, float4* __restrict__ adam_m, float4* __restrict__ adam_v,
     const uint32_t* __restrict__ skip, const BatchTable* __restrict__ bt, uint2* bf, float* __restrict__ stat_maxg) {
+  chain_begin();
   __shared__ float acc[kPlanes * 4][kBatchBwdThreads];
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -1192,8 +1191,8 @@ Status launch_project_bwd_batch_adam(Ctx* c, float* planes, float* m, float* v, 
   float4* av = reinterpret_cast<float4*>(v);
   uint2* bf = static_cast<uint2*>(bf16);
 #define SPLAT_PBB(D, B)                                                                                          \
-  project_bwd_batch_adam_kernel<D, B><<<grid, kBatchBwdThreads, 0, c->stream>>>(p, n, cap, opts, r, pg, pcap, sa, sd, \
-                                                                                 sm, absgrad, am, av, skip, bt, bf, smg)
+  SPLAT_TRY(launch_chained(c, "project_bwd_batch_adam_kernel", project_bwd_batch_adam_kernel<D, B>, grid, kBatchBwdThreads, 0, p, n, cap, opts, r, pg, pcap, sa, sd, \
+                                                                                 sm, absgrad, am, av, skip, bt, bf, smg))
   if (bf) {
     switch (opts.sh_degree) {
       case 0: SPLAT_PBB(0, true); break;
@@ -1210,8 +1209,6 @@ Status launch_project_bwd_batch_adam(Ctx* c, float* planes, float* m, float* v, 
     }
   }
 #undef SPLAT_PBB
-  c->launches.count++;
-  SPLAT_LAUNCHED("project_bwd_batch_adam_kernel");
   return Status::ok();
 }
 
@@ -1243,10 +1240,8 @@ Status launch_params_from_aos(Ctx* c, const float* aos, int64_t n, float* planes
 
 Status launch_params_to_aos(Ctx* c, const float* planes, int64_t n, int64_t cap, float* aos) {
   if (n == 0) return Status::ok();
-  planes_to_aos_kernel<<<ceil_div(n, kConvG), kConvG, 0, c->stream>>>(reinterpret_cast<const float4*>(planes), n, cap,
-                                                                      aos);
-  c->launches.count++;
-  SPLAT_LAUNCHED("planes_to_aos_kernel");
+  SPLAT_TRY(launch_chained(c, "planes_to_aos_kernel", planes_to_aos_kernel, ceil_div(n, kConvG), kConvG, 0,
+                           reinterpret_cast<const float4*>(planes), n, cap, aos));
   return Status::ok();
 }
 

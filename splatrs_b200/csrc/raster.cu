@@ -497,6 +497,7 @@ __global__ void __launch_bounds__(32 * FwdShape<TW, TH>::kWarps, 32 / FwdShape<T
   extern __shared__ __align__(16) unsigned char raster_smem[];
   FwdSmem<TW, TH>& sm = *reinterpret_cast<FwdSmem<TW, TH>*>(raster_smem);
   for (int i = threadIdx.x; i < crm::kExpGridEntries; i += 32 * Shape::kWarps) sm.tab[i] = kExpGrid.v[i];
+  chain_begin();  // the table is constant: it loads while the predecessor drains
   __syncthreads();
   const double* tab = sm.tab;
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -686,6 +687,7 @@ __global__ void __launch_bounds__(TW * TH / PPL, (PPL == 1 ? 1024 : 768) / (TW *
     const float* __restrict__ final_t, const uint32_t* __restrict__ n_contrib, const float* __restrict__ dimage,
     float4* __restrict__ pgrad, int64_t cap, unsigned long long* __restrict__ pairs,
     const BatchTable* __restrict__ bt) {
+  chain_begin();
   typedef TileGeo<TW, TH> Geo;
   constexpr int NT = TW * TH / PPL, NW = NT / 32, WX = TW / 8, SBH = 4 * PPL;
   typedef typename std::conditional<(NW > 8), uint16_t, uint8_t>::type WarpMask;
@@ -1021,6 +1023,7 @@ __global__ void __launch_bounds__(32 * BwdShape<TW, TH>::kWarps, kSmWarps / BwdS
     const float* __restrict__ final_t, const uint32_t* __restrict__ n_contrib, const float* __restrict__ dimage,
     float4* __restrict__ pgrad, int64_t cap, unsigned long long* __restrict__ pairs,
     const BatchTable* __restrict__ bt) {
+  chain_begin();
   typedef BwdShape<TW, TH> Shape;
   typedef typename Shape::W W;
   extern __shared__ __align__(16) unsigned char raster_smem[];
@@ -1542,10 +1545,8 @@ static Status launch_walk(Ctx* c, void (*kernel)(P...), uint32_t tiles, A... arg
       ready.insert(key);
     }
   }
-  kernel<<<ceil_div(tiles, Shape::kTiles), 32 * Shape::kWarps, sizeof(Smem), c->stream>>>(args...);
-  c->launches.count++;
-  SPLAT_LAUNCHED("compositing kernel");
-  return Status::ok();
+  return launch_chained(c, "compositing kernel", kernel, ceil_div(tiles, Shape::kTiles), 32 * Shape::kWarps, sizeof(Smem),
+                        args...);
 }
 
 Status launch_raster_fwd(Ctx* c, const float* proj, const uint32_t* gauss, const uint32_t* ranges, uint32_t width,
@@ -1585,10 +1586,10 @@ Status launch_raster_bwd(Ctx* c, const float* proj, const uint32_t* gauss, const
   const uint32_t blocks = bt ? tiles_cap : rc.tiles(width, height);
   if (blocks == 0) return Status::ok();
 #define SPLAT_BWD(TW, TH, CH, P)                                                                                  \
-  raster_bwd_kernel<TW, TH, CH, P><<<blocks, TW * TH / P, 0, c->stream>>>(                                       \
+  SPLAT_TRY(launch_chained(c, "raster_bwd_kernel", raster_bwd_kernel<TW, TH, CH, P>, blocks, TW * TH / P, 0, \
       reinterpret_cast<const float4*>(proj), gauss, reinterpret_cast<const uint2*>(ranges), width, height, tiles_x, \
       bg[0], bg[1], bg[2], final_t, n_contrib, dimage, reinterpret_cast<float4*>(pgrad), cap,                     \
-      reinterpret_cast<unsigned long long*>(pairs), bt)
+      reinterpret_cast<unsigned long long*>(pairs), bt))
 #define SPLAT_BWD1(TW, TH, CH) SPLAT_BWD(TW, TH, CH, 1)
 #define SPLAT_BWD2X(TW, TH, K, R)                                                                                   \
   SPLAT_TRY((launch_walk<BwdShape<TW, TH>, BwdSmem<TW, TH>>(                                                     \
@@ -1620,8 +1621,6 @@ Status launch_raster_bwd(Ctx* c, const float* proj, const uint32_t* gauss, const
 #undef SPLAT_BWD2X
 #undef SPLAT_BWD1
 #undef SPLAT_BWD
-  c->launches.count++;
-  SPLAT_LAUNCHED("raster_bwd_kernel");
   return Status::ok();
 }
 

@@ -80,6 +80,7 @@ __device__ __forceinline__ uint64_t block_exclusive_u64(uint64_t v, uint64_t* sh
 
 __global__ void __launch_bounds__(kScanThreads) scan_reduce_kernel(const uint32_t* __restrict__ in, int64_t n,
                                                                    uint64_t* __restrict__ partial) {
+  chain_begin();
   __shared__ uint64_t sh[33];
   const int64_t base = (int64_t)blockIdx.x * kScanTile;
   uint64_t s = 0;
@@ -95,6 +96,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_reduce_kernel(const uint32_
 // Single block: exclusive scan of `m` partials in place; total to *total.
 __global__ void __launch_bounds__(1024) scan_partials_kernel(uint64_t* __restrict__ partial, int64_t m,
                                                              uint64_t* __restrict__ total) {
+  chain_begin();
   __shared__ uint64_t sh[33];
   uint64_t carry = 0;
   for (int64_t base = 0; base < m; base += blockDim.x) {
@@ -117,6 +119,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(const uint32_t
                                                                   uint64_t* __restrict__ total,
                                                                   uint32_t* __restrict__ out, int write_total,
                                                                   volatile uint64_t* host_total) {
+  chain_begin();
   __shared__ uint64_t sh[33];
   __shared__ uint64_t before;
   uint64_t first = 0;
@@ -178,16 +181,16 @@ __global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(const uint32_t
 }
 
 // The visible depths' range before a projection: (smallest, largest) = (0xffffffff, 0).
-__global__ void reset_range_kernel(uint32_t* __restrict__ range) { range[threadIdx.x] = threadIdx.x ? 0u : 0xffffffffu; }
+__global__ void reset_range_kernel(uint32_t* __restrict__ range) {
+  chain_begin(); range[threadIdx.x] = threadIdx.x ? 0u : 0xffffffffu; }
 
 Status launch_reset_range(Ctx* c, uint32_t* range) {
-  reset_range_kernel<<<1, 2, 0, c->stream>>>(range);
-  c->launches.count++;
-  SPLAT_LAUNCHED("reset_range_kernel");
+  SPLAT_TRY(launch_chained(c, "reset_range_kernel", reset_range_kernel, 1, 2, 0, range));
   return Status::ok();
 }
 
 __global__ void fill_u32_kernel(uint32_t* __restrict__ dst, size_t words, uint32_t value, int vector) {
+  chain_begin();
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   const size_t quads = vector ? words / 4 : 0;
   uint4* d4 = reinterpret_cast<uint4*>(dst);
@@ -199,6 +202,7 @@ __global__ void fill_u32_kernel(uint32_t* __restrict__ dst, size_t words, uint32
 // Zeroes up to three regions of 32-bit words in one launch.
 __global__ void zero3_u32_kernel(uint32_t* __restrict__ a, size_t na, uint32_t* __restrict__ b, size_t nb,
                                  uint32_t* __restrict__ c3, size_t nc) {
+  chain_begin();
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < na + nb + nc; i += stride) {
     if (i < na)
@@ -214,10 +218,8 @@ Status launch_zero3_u32(Ctx* c, void* a, size_t na, void* b, size_t nb, void* c3
   const size_t words = na + nb + nc;
   if (words == 0) return Status::ok();
   const uint32_t grid = (uint32_t)std::min<size_t>((words + 255) / 256, (size_t)c->sm_count * 8);
-  zero3_u32_kernel<<<grid, 256, 0, c->stream>>>(static_cast<uint32_t*>(a), na, static_cast<uint32_t*>(b), nb,
-                                                static_cast<uint32_t*>(c3), nc);
-  c->launches.count++;
-  SPLAT_LAUNCHED("zero3_u32_kernel");
+  SPLAT_TRY(launch_chained(c, "zero3_u32_kernel", zero3_u32_kernel, grid, 256, 0, static_cast<uint32_t*>(a), na,
+                           static_cast<uint32_t*>(b), nb, static_cast<uint32_t*>(c3), nc));
   return Status::ok();
 }
 
@@ -226,14 +228,14 @@ Status launch_fill_u32(Ctx* c, void* dst, size_t words, uint32_t value) {
   const int vector = (reinterpret_cast<uintptr_t>(dst) & 15u) == 0;
   const size_t items = vector ? (words + 3) / 4 : words;
   const uint32_t grid = (uint32_t)std::min<size_t>((items + 255) / 256, (size_t)c->sm_count * 8);
-  fill_u32_kernel<<<grid, 256, 0, c->stream>>>(reinterpret_cast<uint32_t*>(dst), words, value, vector);
-  c->launches.count++;
-  SPLAT_LAUNCHED("fill_u32_kernel");
+  SPLAT_TRY(launch_chained(c, "fill_u32_kernel", fill_u32_kernel, grid, 256, 0, reinterpret_cast<uint32_t*>(dst),
+                           words, value, vector));
   return Status::ok();
 }
 
 __global__ void publish_u32_kernel(const uint32_t* __restrict__ a, int na, const uint32_t* __restrict__ b, int nb,
                                    volatile uint32_t* out) {
+  chain_begin();
   const int lane = threadIdx.x;
   if (lane < na) out[lane] = a[lane];
   if (lane < nb) out[na + lane] = b[lane];
@@ -241,14 +243,14 @@ __global__ void publish_u32_kernel(const uint32_t* __restrict__ a, int na, const
 }
 
 __global__ void load_words_kernel(const volatile uint32_t* src, uint32_t* __restrict__ dst, int words) {
+  chain_begin();
   for (int i = threadIdx.x; i < words; i += 32) dst[i] = src[i];
 }
 
 Status launch_load_words(Ctx* c, const void* src_mapped_dev, void* dst, int words) {
-  load_words_kernel<<<1, 32, 0, c->stream>>>(static_cast<const volatile uint32_t*>(src_mapped_dev),
-                                             static_cast<uint32_t*>(dst), words);
-  c->launches.count++;
-  SPLAT_LAUNCHED("load_words_kernel");
+  SPLAT_TRY(launch_chained(c, "load_words_kernel", load_words_kernel, 1, 32, 0,
+                           static_cast<const volatile uint32_t*>(src_mapped_dev), static_cast<uint32_t*>(dst),
+                           words));
   return Status::ok();
 }
 
@@ -258,9 +260,8 @@ Status launch_publish_u32(Ctx* c, const uint32_t* a, int na, const uint32_t* b, 
 
 Status launch_publish_u32_to(Ctx* c, const uint32_t* a, int na, const uint32_t* b, int nb, void* out_dev) {
   if (na < 0 || nb < 0 || na + nb > 32) return Status::make(SPLAT_ERR_INVALID, "publish: at most 32 words");
-  publish_u32_kernel<<<1, 32, 0, c->stream>>>(a, na, b, nb, reinterpret_cast<volatile uint32_t*>(out_dev));
-  c->launches.count++;
-  SPLAT_LAUNCHED("publish_u32_kernel");
+  SPLAT_TRY(launch_chained(c, "publish_u32_kernel", publish_u32_kernel, 1, 32, 0, a, na, b, nb,
+                           reinterpret_cast<volatile uint32_t*>(out_dev)));
   return Status::ok();
 }
 
@@ -276,16 +277,13 @@ Status launch_scan_u32_into(Ctx* c, const uint32_t* in, int64_t n, uint32_t* out
   const uint32_t blocks = ceil_div((uint64_t)std::max<int64_t>(n, 1), kScanTile);
   const int scanned = blocks > kScanDirect;
   if (blocks > 1) {
-    scan_reduce_kernel<<<blocks, kScanThreads, 0, c->stream>>>(in, n, partial);
-    c->launches.count++;
+    SPLAT_TRY(launch_chained(c, "scan_reduce_kernel", scan_reduce_kernel, blocks, kScanThreads, 0, in, n, partial));
   }
   if (scanned) {
-    scan_partials_kernel<<<1, 1024, 0, c->stream>>>(partial, blocks, total);
-    c->launches.count++;
+    SPLAT_TRY(launch_chained(c, "scan_partials_kernel", scan_partials_kernel, 1, 1024, 0, partial, blocks, total));
   }
-  scan_apply_kernel<<<blocks, kScanThreads, 0, c->stream>>>(in, n, partial, scanned, total, out, write_total, host_total);
-  c->launches.count++;
-  SPLAT_LAUNCHED("scan kernels");
+  SPLAT_TRY(launch_chained(c, "scan_apply_kernel", scan_apply_kernel, blocks, kScanThreads, 0, in, n, partial,
+                           scanned, total, out, write_total, host_total));
   return Status::ok();
 }
 
@@ -412,6 +410,7 @@ __global__ void __launch_bounds__(256) emit_keys_kernel(const float4* __restrict
                                                         uint32_t tiles_x, const uint32_t* __restrict__ depth_range,
                                                         KeyLayout lay, uint64_t* __restrict__ keys,
                                                         uint32_t* __restrict__ vals, uint32_t* __restrict__ hist) {
+  chain_begin();
   emit_keys_body<kPacked>(rec, entry_offset, n, tiles_x, depth_range, lay, lay.E, keys, vals, hist, nullptr, 1);
 }
 
@@ -684,6 +683,7 @@ __global__ void __launch_bounds__(S::kThreads) radix_onesweep_kernel(const uint6
                                                                      const uint32_t* __restrict__ vals_in, int64_t n,
                                                                      int pass, SortCtl ctl, uint32_t* __restrict__ err,
                                                                      PassOut out) {
+  chain_begin();
   extern __shared__ __align__(16) unsigned char dsm[];
   const uint64_t tiles = (uint64_t)((n + S::kTile - 1) / S::kTile);
   onesweep_body<S, kPacked, W>(keys_in, vals_in, n, 8 * pass + out.vbits, ctl.hist + 256 * pass,
@@ -726,6 +726,7 @@ __device__ __forceinline__ void tile_ranges_body(const uint32_t* __restrict__ ti
 }
 __global__ void __launch_bounds__(kRangeThreads) tile_ranges_kernel(const uint32_t* __restrict__ tiles, int64_t n,
                                                                     uint32_t* __restrict__ ranges) {
+  chain_begin();
   tile_ranges_body(tiles, n, ranges);
 }
 
@@ -742,10 +743,7 @@ static Status launch_pass(Ctx* c, void (*kernel)(P...), size_t smem, uint64_t ti
       ready.insert(key);
     }
   }
-  kernel<<<(uint32_t)tiles, S::kThreads, smem, c->stream>>>(args...);
-  c->launches.count++;
-  SPLAT_LAUNCHED("radix_onesweep_kernel");
-  return Status::ok();
+  return launch_chained(c, "radix_onesweep_kernel", kernel, (uint32_t)tiles, S::kThreads, smem, args...);
 }
 
 template <bool kPacked, typename W>
@@ -766,11 +764,9 @@ static Status sort_entries(Ctx* c, const float* proj, const uint32_t* entry_offs
   const SortCtl ctl = carve_sort_ctl(ctl_base, E);
   SPLAT_TRY(launch_zero3_u32(c, ranges, (size_t)num_tiles * 2, ctl.status, status_bytes(E, lay.passes) / 4, ctl.hist,
                              kSortCounterWords));
-  emit_keys_kernel<kPacked><<<emit_blocks(c, n), 256, 0, c->stream>>>(reinterpret_cast<const float4*>(proj),
-                                                                      entry_offset, n, tiles_x, depth_range, lay, ka,
-                                                                      va, ctl.hist);
-  c->launches.count++;
-  SPLAT_LAUNCHED("emit_keys_kernel");
+  SPLAT_TRY(launch_chained(c, "emit_keys_kernel", emit_keys_kernel<kPacked>, emit_blocks(c, n), 256, 0,
+                           reinterpret_cast<const float4*>(proj), entry_offset, n, tiles_x, depth_range, lay, ka, va,
+                           ctl.hist));
   uint32_t* err = reinterpret_cast<uint32_t*>(static_cast<char*>(c->host_small_dev) + kAsyncErrorWordOffset);
   for (int p = 0; p < lay.passes; p++) {
     PassOut out{};
@@ -795,9 +791,8 @@ static Status sort_entries(Ctx* c, const float* proj, const uint32_t* entry_offs
     std::swap(ka, kb);
     std::swap(va, vb);
   }
-  tile_ranges_kernel<<<ceil_div(E, 4 * kRangeThreads), kRangeThreads, 0, c->stream>>>(reinterpret_cast<const uint32_t*>(ka), E, ranges);
-  c->launches.count++;
-  SPLAT_LAUNCHED("tile_ranges_kernel");
+  SPLAT_TRY(launch_chained(c, "tile_ranges_kernel", tile_ranges_kernel, ceil_div(E, 4 * kRangeThreads),
+                           kRangeThreads, 0, reinterpret_cast<const uint32_t*>(ka), E, ranges));
   return Status::ok();
 }
 
@@ -854,6 +849,7 @@ __global__ void __launch_bounds__(256) emit_keys_dev_kernel(
     const uint32_t* __restrict__ depth_range, const uint64_t* __restrict__ E_dev, int64_t E_cap, int tbits, int vbits,
     uint64_t* __restrict__ keys, uint32_t* __restrict__ vals, uint32_t* __restrict__ hist,
     uint32_t* __restrict__ overflow, const BatchTable* __restrict__ bt, int64_t n_view) {
+  chain_begin();
   const KeyLayout lay = dev_layout(E_dev, E_cap, depth_range, tbits, vbits);
   if (blockIdx.x == 0 && threadIdx.x == 0 && *E_dev > (uint64_t)E_cap) atomicOr(overflow, 1u);
   emit_keys_body<kPacked>(rec, entry_offset, n, tiles_x, depth_range, lay, E_cap, keys, vals, hist, bt, n_view);
@@ -868,6 +864,7 @@ template <typename S, bool kPacked, typename W>
 __global__ void __launch_bounds__(S::kThreads) radix_onesweep_dev_kernel(
     DevBuffers b, const uint64_t* __restrict__ E_dev, int64_t E_cap, const uint32_t* __restrict__ dr, int tbits,
     int vbits, int pass, SortCtl ctl, uint64_t tiles_cap, uint32_t* __restrict__ err, uint32_t* __restrict__ vals_final) {
+  chain_begin();
   extern __shared__ __align__(16) unsigned char dsm[];
   const KeyLayout lay = dev_layout(E_dev, E_cap, dr, tbits, vbits);
   if (pass >= lay.passes) return;
@@ -887,6 +884,7 @@ __global__ void __launch_bounds__(S::kThreads) radix_onesweep_dev_kernel(
 __global__ void __launch_bounds__(kRangeThreads) tile_ranges_dev_kernel(DevBuffers b, const uint64_t* __restrict__ E_dev,
                                                                         int64_t E_cap, const uint32_t* __restrict__ dr,
                                                                         int tbits, uint32_t* __restrict__ ranges) {
+  chain_begin();
   const KeyLayout lay = dev_layout(E_dev, E_cap, dr, tbits, 0);
   // The tiles are where the last pass would have written keys.
   tile_ranges_body(reinterpret_cast<const uint32_t*>((lay.passes - 1) & 1 ? b.ka : b.kb), lay.E, ranges);
@@ -922,11 +920,9 @@ static Status sort_entries_dev(Ctx* c, const float* proj, const uint32_t* entry_
   SPLAT_TRY(launch_zero3_u32(c, ranges, (size_t)num_tiles * 2, ctl.status, status_bytes(cap, max_passes) / 4, ctl.hist,
                              kSortCounterWords));
   if (n > 0) {
-    emit_keys_dev_kernel<kPacked><<<emit_blocks(c, n), 256, 0, c->stream>>>(
-        reinterpret_cast<const float4*>(proj), entry_offset, n, tiles_x, dr, E_dev, E_cap, tbits, vbits, b.ka, b.va,
-        ctl.hist, overflow, bt, n_view);
-    c->launches.count++;
-    SPLAT_LAUNCHED("emit_keys_dev_kernel");
+    SPLAT_TRY(launch_chained(c, "emit_keys_dev_kernel", emit_keys_dev_kernel<kPacked>, emit_blocks(c, n), 256, 0,
+                             reinterpret_cast<const float4*>(proj), entry_offset, n, tiles_x, dr, E_dev, E_cap,
+                             tbits, vbits, b.ka, b.va, ctl.hist, overflow, bt, n_view));
   }
   for (int pass = 0; pass < max_passes; pass++) {
 #define SPLAT_PASS(S)                                                                                          \
@@ -940,9 +936,8 @@ static Status sort_entries_dev(Ctx* c, const float* proj, const uint32_t* entry_
       SPLAT_PASS(SortLarge);
 #undef SPLAT_PASS
   }
-  tile_ranges_dev_kernel<<<ceil_div(cap, 4 * kRangeThreads), kRangeThreads, 0, c->stream>>>(b, E_dev, E_cap, dr, tbits, ranges);
-  c->launches.count++;
-  SPLAT_LAUNCHED("tile_ranges_dev_kernel");
+  SPLAT_TRY(launch_chained(c, "tile_ranges_dev_kernel", tile_ranges_dev_kernel, ceil_div(cap, 4 * kRangeThreads),
+                           kRangeThreads, 0, b, E_dev, E_cap, dr, tbits, ranges));
   return Status::ok();
 }
 
