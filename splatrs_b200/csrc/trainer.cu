@@ -1185,14 +1185,7 @@ SPLAT_API int splat_trainer_get_model(splat_trainer* t, float* aos59_host) {
   if (!t || (!aos59_host && t->n)) return SPLAT_ERR_INVALID;
   TEnter e(t);
   Ctx* c = t->c;
-  DevBuf tmp;
-  Status s = tmp.ensure((size_t)std::max<int64_t>(t->n, 1) * 59 * 4);
-  if (s.good()) s = launch_params_to_aos(c, t->cur.params.as<float>(), t->n, t->cur.cap, tmp.as<float>());
-  if (s.good() && t->n)
-    s = cuda_status(cudaMemcpyAsync(aos59_host, tmp.ptr, (size_t)t->n * 59 * 4, cudaMemcpyDeviceToHost, c->stream),
-                    "download model");
-  if (s.good()) s = cuda_status(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");
-  tmp.release();
+  const Status s = download_records(c, t->cur.params.as<float>(), t->n, t->cur.cap, aos59_host);
   return s.good() ? SPLAT_OK : tfail(t, s);
 }
 
@@ -1202,17 +1195,8 @@ SPLAT_API int splat_trainer_get_moments(splat_trainer* t, float* m_aos59_host, f
   if (!t || (t->n && (!m_aos59_host || !v_aos59_host))) return SPLAT_ERR_INVALID;
   TEnter e(t);
   Ctx* c = t->c;
-  DevBuf tmp;
-  Status s = tmp.ensure((size_t)std::max<int64_t>(t->n, 1) * 59 * 4);
-  for (int k = 0; k < 2 && s.good(); k++) {
-    s = launch_params_to_aos(c, (k ? t->cur.v : t->cur.m).as<float>(), t->n, t->cur.cap, tmp.as<float>());
-    if (s.good() && t->n)
-      s = cuda_status(cudaMemcpyAsync(k ? v_aos59_host : m_aos59_host, tmp.ptr, (size_t)t->n * 59 * 4,
-                                      cudaMemcpyDeviceToHost, c->stream),
-                      "download moments");
-    if (s.good()) s = cuda_status(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize");
-  }
-  tmp.release();
+  Status s = download_records(c, t->cur.m.as<float>(), t->n, t->cur.cap, m_aos59_host);
+  if (s.good()) s = download_records(c, t->cur.v.as<float>(), t->n, t->cur.cap, v_aos59_host);
   return s.good() ? SPLAT_OK : tfail(t, s);
 }
 
