@@ -997,10 +997,10 @@ Status launch_project_fwd(Ctx* c, const float* planes, int64_t n, int64_t cap, c
   const float4* p = reinterpret_cast<const float4*>(planes);
   float4* r = reinterpret_cast<float4*>(proj);
   const uint2* bf = static_cast<const uint2*>(bf16);
-#define SPLAT_PFWD(D, B) \
-  SPLAT_TRY(launch_chained(c, "project_fwd_kernel", project_fwd_kernel<D, B>, dim3(grid, bt ? kMaxViews : 1), bs, 0, p, n, cap, cam, opts, r, num_tiles, \
-                                                                                 depth_range, sp, bf, bt, \
-                                                                                 c->raster.tile_w, c->raster.tile_h))
+#define SPLAT_PFWD(D, B)                                                                                             \
+  SPLAT_TRY(launch_chained(c, "project_fwd_kernel", project_fwd_kernel<D, B>, dim3(grid, bt ? kMaxViews : 1), bs, 0, \
+                           p, n, cap, cam, opts, r, num_tiles, depth_range, sp, bf, bt, c->raster.tile_w,            \
+                           c->raster.tile_h))
   if (bf) {
     switch (opts.sh_degree) {
       case 0: SPLAT_PFWD(0, true); break;
@@ -1062,7 +1062,7 @@ static Status project_bwd_launch(Ctx* c, const float* planes, int64_t n, int64_t
     if (with_maxg) smg = reinterpret_cast<float*>(sm + cap);
   }
 #define SPLAT_PBWD(D) \
-  SPLAT_TRY(launch_chained(c, "project_bwd_kernel", project_bwd_kernel<D, ADAM, BF16>, grid, bs, 0, p, n, cap, cam,
+  SPLAT_TRY(launch_chained(c, "project_bwd_kernel", project_bwd_kernel<D, ADAM, BF16>, grid, bs, 0, p, n, cap, cam, \
                            opts, r, pg, o, sa, sd, sm, absgrad, am, av, adam, skip, sp, bf, smg))
   switch (opts.sh_degree) {
     case 0: SPLAT_PBWD(0); break;
@@ -1190,9 +1190,10 @@ Status launch_project_bwd_batch_adam(Ctx* c, float* planes, float* m, float* v, 
   float4* am = reinterpret_cast<float4*>(m);
   float4* av = reinterpret_cast<float4*>(v);
   uint2* bf = static_cast<uint2*>(bf16);
-#define SPLAT_PBB(D, B)                                                                                          \
-  SPLAT_TRY(launch_chained(c, "project_bwd_batch_adam_kernel", project_bwd_batch_adam_kernel<D, B>, grid, kBatchBwdThreads, 0, p, n, cap, opts, r, pg, pcap, sa, sd, \
-                                                                                 sm, absgrad, am, av, skip, bt, bf, smg))
+#define SPLAT_PBB(D, B)                                                                                         \
+  SPLAT_TRY(launch_chained(c, "project_bwd_batch_adam_kernel", project_bwd_batch_adam_kernel<D, B>, grid,        \
+                           kBatchBwdThreads, 0, p, n, cap, opts, r, pg, pcap, sa, sd, sm, absgrad, am, av, skip, \
+                           bt, bf, smg))
   if (bf) {
     switch (opts.sh_degree) {
       case 0: SPLAT_PBB(0, true); break;

@@ -1545,8 +1545,8 @@ static Status launch_walk(Ctx* c, void (*kernel)(P...), uint32_t tiles, A... arg
       ready.insert(key);
     }
   }
-  return launch_chained(c, "compositing kernel", kernel, ceil_div(tiles, Shape::kTiles), 32 * Shape::kWarps, sizeof(Smem),
-                        args...);
+  return launch_chained(c, "compositing kernel", kernel, ceil_div(tiles, Shape::kTiles), 32 * Shape::kWarps,
+                        sizeof(Smem), args...);
 }
 
 Status launch_raster_fwd(Ctx* c, const float* proj, const uint32_t* gauss, const uint32_t* ranges, uint32_t width,
