@@ -152,11 +152,15 @@ __host__ __device__ __forceinline__ uint32_t sat_u32(float v) {
 // way chain_begin does nothing. Twelve small kernels of a 256x256 view 110 -> 94 us, 100k Gaussians
 // at 1280x720 with gradients 259 -> 233, 1M at 1920x1080 1,606 -> 1,592. Under capture launches stay
 // ordinary ones: a graph of them replays faster than one with these edges (a 20-kernel training
-// iteration 234 against 294 us).
+// iteration 234 against 294 us). The compositing kernels only wait and let no successor in before
+// they end: blocks that came early would take places on the SMs beside unfinished ones, and a
+// kernel whose blocks all fit at once would be spread unevenly (34k Gaussians at 256x256 backward
+// 88 -> 101 us after another compositing kernel).
 #if defined(__CUDACC__)
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_begin() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  chain_wait();
 }
 template <typename... P, typename... A>
 inline Status launch_chained(Ctx* c, const char* what, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,

@@ -497,7 +497,7 @@ __global__ void __launch_bounds__(32 * FwdShape<TW, TH>::kWarps, 32 / FwdShape<T
   extern __shared__ __align__(16) unsigned char raster_smem[];
   FwdSmem<TW, TH>& sm = *reinterpret_cast<FwdSmem<TW, TH>*>(raster_smem);
   for (int i = threadIdx.x; i < crm::kExpGridEntries; i += 32 * Shape::kWarps) sm.tab[i] = kExpGrid.v[i];
-  chain_begin();  // the table is constant: it loads while the predecessor drains
+  chain_wait();  // the table is constant: it loads while the predecessor drains
   __syncthreads();
   const double* tab = sm.tab;
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -687,7 +687,7 @@ __global__ void __launch_bounds__(TW * TH / PPL, (PPL == 1 ? 1024 : 768) / (TW *
     const float* __restrict__ final_t, const uint32_t* __restrict__ n_contrib, const float* __restrict__ dimage,
     float4* __restrict__ pgrad, int64_t cap, unsigned long long* __restrict__ pairs,
     const BatchTable* __restrict__ bt) {
-  chain_begin();
+  chain_wait();
   typedef TileGeo<TW, TH> Geo;
   constexpr int NT = TW * TH / PPL, NW = NT / 32, WX = TW / 8, SBH = 4 * PPL;
   typedef typename std::conditional<(NW > 8), uint16_t, uint8_t>::type WarpMask;
@@ -905,8 +905,8 @@ constexpr float kSigmaEdge = 1e-4f;
 // each scalar duplicated, a 13-shuffle reduction of 12 slots over the warp for every entry)
 // this takes about 130 instead of 185 warp instructions per entry. Bound by latency and issue
 // (63% of the issue slots, FMA pipe 48%, shared-memory reads 60%; DRAM 3% of its peak).
-// Time: 1M Gaussians at 1920x1080 975 -> 677 us, 187k clustered at 1297x840 377 -> 265, 34k at
-// 256x256 164 -> 88, 20k wide ones at 1386x1080 163 -> 118. kCount adds the evaluated-pair
+// Time: 1M Gaussians at 1920x1080 975 -> 653 us, 187k clustered at 1297x840 377 -> 256, 34k at
+// 256x256 164 -> 78, 20k wide ones at 1386x1080 163 -> 115. kCount adds the evaluated-pair
 // counter (untimed diagnostics only).
 constexpr int kGroup = 8;      // entries per round of the three phases
 constexpr int kBwdStage = 16;  // entries staged per copy
@@ -984,37 +984,55 @@ __device__ __forceinline__ void evaluate_row(BwdStage& st, uint32_t e, uint32_t 
 // State of a lane's two pixels in the reverse walk.
 struct PixelPair {
   f2 T, nbg, d0, d1, d2, acc_r, acc_g, acc_b;
-  // Takes an entry: `g` is its gauss on entry and h on return, `w` alpha T.
-  __device__ __forceinline__ void step(float4 color, float2& g, float2& w) {
-    f2 gauss = f2_make(g.x, g.y);
-    f2 alpha = f2_mul(f2_splat(color.x), gauss);
-    if (!(color.x < SPLAT_ALPHA_MAX)) {
-      // Opacity >= 0.99 (uniform over the warp): alpha clamps at 0.99 and the gradients through
-      // sigma and opacity vanish there (rasterize.rs:414-432).
+};
+
+// Phase 2 of a group: st.h holds gauss on entry and h on return, st.w alpha T. An
+// entry that no pixel of the sub-block takes has gauss 0 and colour 0 and leaves the state as it
+// is. First everything that does not depend on the state, for all entries at once, then the chain
+// through it. kClamp: an opacity may reach 0.99, where alpha clamps and the gradients through
+// sigma and opacity vanish (rasterize.rs:414-432). One branch-free body for eight entries: 677 -> 653
+// us on 1M Gaussians at 1920x1080 against a branch around each entry (four entries at a time: no gain).
+template <bool kClamp>
+__device__ __forceinline__ void walk_entries(BwdStage& st, uint32_t lane, PixelPair& p) {
+  f2 gauss[kGroup], alpha[kGroup], inv[kGroup];
+#pragma unroll
+  for (int k = 0; k < kGroup; k++) {
+    const float2 g = st.h[k][lane];
+    const float opacity = st.color[k].x;
+    gauss[k] = f2_make(g.x, g.y);
+    alpha[k] = f2_mul(f2_splat(opacity), gauss[k]);
+    if (kClamp) {
       float a0, a1;
-      f2_split(alpha, a0, a1);
-      gauss = f2_make(a0 < SPLAT_ALPHA_MAX ? g.x : 0.0f, a1 < SPLAT_ALPHA_MAX ? g.y : 0.0f);
-      alpha = f2_make(fminf(a0, SPLAT_ALPHA_MAX), fminf(a1, SPLAT_ALPHA_MAX));
+      f2_split(alpha[k], a0, a1);
+      gauss[k] = f2_make(a0 < SPLAT_ALPHA_MAX ? g.x : 0.0f, a1 < SPLAT_ALPHA_MAX ? g.y : 0.0f);
+      alpha[k] = f2_make(fminf(a0, SPLAT_ALPHA_MAX), fminf(a1, SPLAT_ALPHA_MAX));
     }
     // Values only from here on (fused, reciprocal for division).
     float o0, o1;
-    f2_split(f2_sub(f2_splat(1.0f), alpha), o0, o1);
-    const f2 inv = f2_make(rcp_fast(o0), rcp_fast(o1));
-    T = f2_mul(T, inv);
-    const f2 dr = f2_sub(f2_splat(color.y), acc_r);
-    const f2 dg = f2_sub(f2_splat(color.z), acc_g);
-    const f2 db = f2_sub(f2_splat(color.w), acc_b);
-    f2 dalpha = f2_fma(db, d2, f2_fma(dg, d1, f2_mul(dr, d0)));
+    f2_split(f2_sub(f2_splat(1.0f), alpha[k]), o0, o1);
+    inv[k] = f2_make(rcp_fast(o0), rcp_fast(o1));
+  }
+#pragma unroll
+  for (int k = 0; k < kGroup; k++) {
+    const float4 color = st.color[k];
+    p.T = f2_mul(p.T, inv[k]);
+    const f2 dr = f2_sub(f2_splat(color.y), p.acc_r);
+    const f2 dg = f2_sub(f2_splat(color.z), p.acc_g);
+    const f2 db = f2_sub(f2_splat(color.w), p.acc_b);
+    f2 dalpha = f2_fma(db, p.d2, f2_fma(dg, p.d1, f2_mul(dr, p.d0)));
     // The accumulator advances right after its use (accum + alpha (c - accum)): the operands
     // of the reference's update on the pixel's next entry.
-    acc_r = f2_fma(alpha, dr, acc_r);
-    acc_g = f2_fma(alpha, dg, acc_g);
-    acc_b = f2_fma(alpha, db, acc_b);
-    dalpha = f2_fma(dalpha, T, f2_mul(nbg, inv));
-    f2_split(f2_mul(gauss, dalpha), g.x, g.y);
-    f2_split(f2_mul(alpha, T), w.x, w.y);
+    p.acc_r = f2_fma(alpha[k], dr, p.acc_r);
+    p.acc_g = f2_fma(alpha[k], dg, p.acc_g);
+    p.acc_b = f2_fma(alpha[k], db, p.acc_b);
+    dalpha = f2_fma(dalpha, p.T, f2_mul(p.nbg, inv[k]));
+    float2 h, w;
+    f2_split(f2_mul(gauss[k], dalpha), h.x, h.y);
+    f2_split(f2_mul(alpha[k], p.T), w.x, w.y);
+    st.h[k][lane] = h;
+    st.w[k][lane] = w;
   }
-};
+}
 
 template <int TW, int TH, bool kCount, int kSmWarps>
 __global__ void __launch_bounds__(32 * BwdShape<TW, TH>::kWarps, kSmWarps / BwdShape<TW, TH>::kWarps) raster_bwd_x2_kernel(
@@ -1023,7 +1041,7 @@ __global__ void __launch_bounds__(32 * BwdShape<TW, TH>::kWarps, kSmWarps / BwdS
     const float* __restrict__ final_t, const uint32_t* __restrict__ n_contrib, const float* __restrict__ dimage,
     float4* __restrict__ pgrad, int64_t cap, unsigned long long* __restrict__ pairs,
     const BatchTable* __restrict__ bt) {
-  chain_begin();
+  chain_wait();
   typedef BwdShape<TW, TH> Shape;
   typedef typename Shape::W W;
   extern __shared__ __align__(16) unsigned char raster_smem[];
@@ -1123,7 +1141,6 @@ __global__ void __launch_bounds__(32 * BwdShape<TW, TH>::kWarps, kSmWarps / BwdS
         const float A = r0.z, B = r0.w, opacity = r1.y, sigma_max = r1.z, sure = sigma_max - kSigmaEdge;
         const f2 dy = f2_sub(pyq, f2_splat(r0.y));
         const f2 cdy = f2_mul(f2_splat(r1.x), dy);
-        if (q == 0) st.color[e] = make_float4(opacity, r1.w, gb.x, gb.y);
         // A row outside the rectangle gets sigma = inf.
         const float inf = __int_as_float(0x7f800000);
         f2 cdyy;
@@ -1187,16 +1204,15 @@ __global__ void __launch_bounds__(32 * BwdShape<TW, TH>::kWarps, kSmWarps / BwdS
         taken |= taken >> 16;
         taken = (taken | (taken >> 8)) & 0xffu;
         if (!taken) continue;
+        const bool clamping = __any_sync(0xffffffffu, clamps);
+        if (q == 0)
+          st.color[e] = (taken >> e) & 1u ? make_float4(opacity, r1.w, gb.x, gb.y) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         __syncwarp();
         // ---- Phase 2
-#pragma unroll
-        for (int k = 0; k < kGroup; k++) {
-          if (!((taken >> k) & 1u)) continue;
-          float2 g = st.h[k][lane], w;
-          pp.step(st.color[k], g, w);
-          st.h[k][lane] = g;
-          st.w[k][lane] = w;
-        }
+        if (clamping)
+          walk_entries<true>(st, lane, pp);
+        else
+          walk_entries<false>(st, lane, pp);
         __syncwarp();
         // ---- Phase 3
         const f2 bdy = f2_mul(f2_splat(B), dy);
@@ -1597,9 +1613,9 @@ Status launch_raster_bwd(Ctx* c, const float* proj, const uint32_t* gauss, const
       reinterpret_cast<const uint2*>(ranges), blocks, width, height, tiles_x, bg[0], bg[1], bg[2], final_t,      \
       n_contrib, dimage, reinterpret_cast<float4*>(pgrad), cap, reinterpret_cast<unsigned long long*>(pairs), bt)))
 // A view whose warps fit the GPU at 16 warps per SM takes the build with 122 registers and no
-// spills, a larger one 20 warps per SM in 96 registers: 34k Gaussians at 256x256 88 us against
-// 97, 2k at 128x96 29 against 31; 1M at 1920x1080 689 against 677, 100k at 1280x720 68 against
-// 66 (both sides of the line within 2% of each other).
+// spills, a larger one 20 warps per SM in 96 registers (measured before phase 2 was branch-free:
+// 34k Gaussians at 256x256 88 us against 97, 2k at 128x96 29 against 31; 1M at 1920x1080 689 against
+// 677, 100k at 1280x720 68 against 66).
 #define SPLAT_BWD2(TW, TH)                                                                                  \
   const bool resident = (uint64_t)blocks * BwdShape<TW, TH>::W::kPerTile <= (uint64_t)c->sm_count * 16;    \
   if (pairs) SPLAT_BWD2X(TW, TH, true, 16); else if (resident) SPLAT_BWD2X(TW, TH, false, 16);            \
