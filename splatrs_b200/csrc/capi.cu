@@ -334,14 +334,16 @@ SPLAT_API int splat_bin_sort(splat_ctx* ctx, const float* proj_dev, const uint32
     return invalid(ctx, "splat_bin_sort: bad buffers");
   Enter e(ctx);
   const volatile uint32_t* h = static_cast<const volatile uint32_t*>(ctx->c.host_small);
-  Status s = launch_publish_u32(&ctx->c, depth_range_dev, 2, nullptr, 0);
+  // The launch that clears the sort's buffers also stores the depth range into mapped host memory.
+  SortBuffers buf;
+  Status s = launch_bin_sort_begin(&ctx->c, n, num_entries, width, height, tile_range_dev, depth_range_dev, &buf);
   if (s.good()) s = cuda_status(cudaStreamSynchronize(ctx->c.stream), "cudaStreamSynchronize");
   if (s.good()) s = take_sort_error(&ctx->c);  // of an earlier sort on this context
   if (!s.good()) return fail(ctx, s);
   const uint32_t dmin = h[0], dmax = h[1];
   if (num_entries > 0 && dmin > dmax) return invalid(ctx, "splat_bin_sort: depth range is empty but entries exist");
   return finish(ctx, launch_bin_sort(&ctx->c, proj_dev, entry_offset_dev, n, num_entries, depth_range_dev, dmin,
-                                     num_entries > 0 ? dmax : dmin, width, height, gauss_dev, keys_dev,
+                                     num_entries > 0 ? dmax : dmin, width, height, buf, gauss_dev, keys_dev,
                                      tile_range_dev));
 }
 

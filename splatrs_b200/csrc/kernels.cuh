@@ -168,9 +168,20 @@ Status launch_publish_u32_to(Ctx* c, const uint32_t* a, int na, const uint32_t* 
 Status launch_scan_u32_into(Ctx* c, const uint32_t* in, int64_t n, uint32_t* out, int write_total,
                             uint64_t* partial, uint64_t* total, uint64_t* host_total = nullptr);
 constexpr int kScanValuesPerBlock = 4096;
+// The sort of E entries in two steps around the read of the depth range: _begin reserves its
+// buffers, clears them and the tile ranges, and stores the two words at `show` (the depth range;
+// may be NULL) at the start of the mapped host page.
+struct SortBuffers {
+  uint64_t *ka = nullptr, *kb = nullptr;
+  uint32_t *va = nullptr, *vb = nullptr;
+  void* ctl = nullptr;
+};
+Status launch_bin_sort_begin(Ctx* c, int64_t n, int64_t E, uint32_t width, uint32_t height, uint32_t* ranges,
+                             const uint32_t* show, SortBuffers* buf);
 Status launch_bin_sort(Ctx* c, const float* proj, const uint32_t* entry_offset, int64_t n, int64_t E,
                        const uint32_t* depth_range_dev, uint32_t depth_min, uint32_t depth_max, uint32_t width,
-                       uint32_t height, uint32_t* gauss_out, uint64_t* keys_out, uint32_t* ranges);
+                       uint32_t height, const SortBuffers& buf, uint32_t* gauss_out, uint64_t* keys_out,
+                       uint32_t* ranges);
 
 // The supported compositing configurations (tile shapes x chunk depths x backward pixels
 // per thread).

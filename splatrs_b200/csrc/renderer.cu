@@ -119,8 +119,10 @@ Status render_view(Ctx* c, const float* planes, int64_t n, int64_t cap, const sp
   const uint64_t drw = h[1];
   const uint32_t drh[2] = {(uint32_t)drw, (uint32_t)(drw >> 32)};
   SPLAT_TRY(v.gauss.ensure((size_t)std::max<uint64_t>(E, 1) * 4));
+  SortBuffers buf;
+  SPLAT_TRY(launch_bin_sort_begin(c, n, (int64_t)E, cam.width, cam.height, v.tile_range.as<uint32_t>(), nullptr, &buf));
   SPLAT_TRY(launch_bin_sort(c, proj, v.entry_offset.as<uint32_t>(), n, (int64_t)E, dr, drh[0],
-                            E > 0 ? drh[1] : drh[0], cam.width, cam.height, v.gauss.as<uint32_t>(), nullptr,
+                            E > 0 ? drh[1] : drh[0], cam.width, cam.height, buf, v.gauss.as<uint32_t>(), nullptr,
                             v.tile_range.as<uint32_t>()));
   SPLAT_TRY(launch_raster_fwd(c, proj, v.gauss.as<uint32_t>(), v.tile_range.as<uint32_t>(), cam.width, cam.height, bg,
                               v.image.as<float>(), v.final_t.as<float>(), v.n_contrib.as<uint32_t>(), nullptr));

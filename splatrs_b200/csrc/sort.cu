@@ -199,10 +199,16 @@ __global__ void fill_u32_kernel(uint32_t* __restrict__ dst, size_t words, uint32
   for (size_t i = quads * 4 + (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < words; i += stride) dst[i] = value;
 }
 
-// Zeroes up to three regions of 32-bit words in one launch.
+// Zeroes up to three regions of 32-bit words in one launch, and stores two words of `show` (may
+// be NULL) into mapped host memory on the way.
 __global__ void zero3_u32_kernel(uint32_t* __restrict__ a, size_t na, uint32_t* __restrict__ b, size_t nb,
-                                 uint32_t* __restrict__ c3, size_t nc) {
+                                 uint32_t* __restrict__ c3, size_t nc, const uint32_t* __restrict__ show,
+                                 volatile uint32_t* host) {
   chain_begin();
+  if (show && blockIdx.x == 0 && threadIdx.x < 2) {
+    host[threadIdx.x] = show[threadIdx.x];
+    __threadfence_system();
+  }
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < na + nb + nc; i += stride) {
     if (i < na)
@@ -214,12 +220,14 @@ __global__ void zero3_u32_kernel(uint32_t* __restrict__ a, size_t na, uint32_t* 
   }
 }
 
-Status launch_zero3_u32(Ctx* c, void* a, size_t na, void* b, size_t nb, void* c3, size_t nc) {
+static Status launch_zero3_u32(Ctx* c, void* a, size_t na, void* b, size_t nb, void* c3, size_t nc,
+                               const uint32_t* show = nullptr) {
   const size_t words = na + nb + nc;
   if (words == 0) return Status::ok();
   const uint32_t grid = (uint32_t)std::min<size_t>((words + 255) / 256, (size_t)c->sm_count * 8);
   SPLAT_TRY(launch_chained(c, "zero3_u32_kernel", zero3_u32_kernel, grid, 256, 0, static_cast<uint32_t*>(a), na,
-                           static_cast<uint32_t*>(b), nb, static_cast<uint32_t*>(c3), nc));
+                           static_cast<uint32_t*>(b), nb, static_cast<uint32_t*>(c3), nc, show,
+                           static_cast<volatile uint32_t*>(c->host_small_dev)));
   return Status::ok();
 }
 
@@ -413,6 +421,9 @@ __global__ void __launch_bounds__(256) emit_keys_kernel(const float4* __restrict
   chain_begin();
   emit_keys_body<kPacked>(rec, entry_offset, n, tiles_x, depth_range, lay, lay.E, keys, vals, hist, nullptr, 1);
 }
+
+// Passes that keys can need: depth bits span 32 bits at most (31 while depths are positive).
+static int max_passes(int tbits) { return (tbits + 32 + 7) / 8; }
 
 // Blocks of an emission over n records.
 static uint32_t emit_blocks(const Ctx* c, int64_t n) {
@@ -748,22 +759,12 @@ static Status launch_pass(Ctx* c, void (*kernel)(P...), size_t smem, uint64_t ti
 
 template <bool kPacked, typename W>
 static Status sort_entries(Ctx* c, const float* proj, const uint32_t* entry_offset, int64_t n, const KeyLayout& lay,
-                           const uint32_t* depth_range, uint32_t depth_min, uint32_t tiles_x, uint32_t num_tiles,
+                           const uint32_t* depth_range, uint32_t depth_min, uint32_t tiles_x, const SortBuffers& buf,
                            uint32_t* gauss_out, uint64_t* keys_out, uint32_t* ranges) {
   const int64_t E = lay.E;
-  uint64_t *ka = nullptr, *kb = nullptr;
-  uint32_t *va = nullptr, *vb = nullptr;
-  SPLAT_TRY(arena_reserve(c, (size_t)E * 8, (void**)&ka));
-  SPLAT_TRY(arena_reserve(c, (size_t)E * 8, (void**)&kb));
-  if (!kPacked) {
-    SPLAT_TRY(arena_reserve(c, (size_t)E * 4, (void**)&va));
-    SPLAT_TRY(arena_reserve(c, (size_t)E * 4, (void**)&vb));
-  }
-  void* ctl_base = nullptr;
-  SPLAT_TRY(arena_reserve(c, sort_ctl_bytes(E), &ctl_base));
-  const SortCtl ctl = carve_sort_ctl(ctl_base, E);
-  SPLAT_TRY(launch_zero3_u32(c, ranges, (size_t)num_tiles * 2, ctl.status, status_bytes(E, lay.passes) / 4, ctl.hist,
-                             kSortCounterWords));
+  uint64_t *ka = buf.ka, *kb = buf.kb;
+  uint32_t *va = buf.va, *vb = buf.vb;
+  const SortCtl ctl = carve_sort_ctl(buf.ctl, E);
   SPLAT_TRY(launch_chained(c, "emit_keys_kernel", emit_keys_kernel<kPacked>, emit_blocks(c, n), 256, 0,
                            reinterpret_cast<const float4*>(proj), entry_offset, n, tiles_x, depth_range, lay, ka, va,
                            ctl.hist));
@@ -796,15 +797,29 @@ static Status sort_entries(Ctx* c, const float* proj, const uint32_t* entry_offs
   return Status::ok();
 }
 
+Status launch_bin_sort_begin(Ctx* c, int64_t n, int64_t E, uint32_t width, uint32_t height, uint32_t* ranges,
+                             const uint32_t* show, SortBuffers* buf) {
+  const uint32_t num_tiles = c->raster.tiles(width, height);
+  if (E == 0) return launch_zero3_u32(c, ranges, (size_t)num_tiles * 2, nullptr, 0, nullptr, 0, show);
+  const int tbits = bits_for(num_tiles);
+  SPLAT_TRY(arena_reserve(c, (size_t)E * 8, (void**)&buf->ka));
+  SPLAT_TRY(arena_reserve(c, (size_t)E * 8, (void**)&buf->kb));
+  if (tbits + 32 + bits_for((uint64_t)n) > 64) {  // keys may turn out too wide to pack
+    SPLAT_TRY(arena_reserve(c, (size_t)E * 4, (void**)&buf->va));
+    SPLAT_TRY(arena_reserve(c, (size_t)E * 4, (void**)&buf->vb));
+  }
+  SPLAT_TRY(arena_reserve(c, sort_ctl_bytes(E), &buf->ctl));
+  const SortCtl ctl = carve_sort_ctl(buf->ctl, E);
+  return launch_zero3_u32(c, ranges, (size_t)num_tiles * 2, ctl.status, status_bytes(E, max_passes(tbits)) / 4,
+                          ctl.hist, kSortCounterWords, show);
+}
+
 Status launch_bin_sort(Ctx* c, const float* proj, const uint32_t* entry_offset, int64_t n, int64_t E,
                        const uint32_t* depth_range_dev, uint32_t depth_min, uint32_t depth_max, uint32_t width,
-                       uint32_t height, uint32_t* gauss_out, uint64_t* keys_out, uint32_t* ranges) {
-  const uint32_t tiles_x = c->raster.tiles_x(width), tiles_y = c->raster.tiles_y(height);
-  const uint32_t num_tiles = tiles_x * tiles_y;
-  if (E == 0) {
-    SPLAT_TRY(launch_fill_u32(c, ranges, (size_t)num_tiles * 2, 0u));
-    return Status::ok();
-  }
+                       uint32_t height, const SortBuffers& buf, uint32_t* gauss_out, uint64_t* keys_out,
+                       uint32_t* ranges) {
+  if (E == 0) return Status::ok();
+  const uint32_t tiles_x = c->raster.tiles_x(width), num_tiles = c->raster.tiles(width, height);
   const int tbits = bits_for(num_tiles), nbits = bits_for((uint64_t)n);
   KeyLayout lay;
   lay.E = E;
@@ -813,8 +828,8 @@ Status launch_bin_sort(Ctx* c, const float* proj, const uint32_t* entry_offset, 
   const bool packed = tbits + lay.dbits + nbits <= 64;
   lay.vbits = packed ? nbits : 0;
 #define SPLAT_SORT(P, W)                                                                                      \
-  sort_entries<P, W>(c, proj, entry_offset, n, lay, depth_range_dev, depth_min, tiles_x, num_tiles, gauss_out, \
-                     keys_out, ranges)
+  sort_entries<P, W>(c, proj, entry_offset, n, lay, depth_range_dev, depth_min, tiles_x, buf, gauss_out, keys_out, \
+                     ranges)
   if (wide_words(E)) return packed ? SPLAT_SORT(true, uint64_t) : SPLAT_SORT(false, uint64_t);
   return packed ? SPLAT_SORT(true, uint32_t) : SPLAT_SORT(false, uint32_t);
 #undef SPLAT_SORT
@@ -827,7 +842,7 @@ Status launch_bin_sort(Ctx* c, const float* proj, const uint32_t* entry_offset, 
 // passes the keys do not need, and the last needed pass writes the caller's buffer. An
 // entry count above E_cap sets *overflow (sticky) and sorts only the first E_cap entries;
 // the caller must discard that view's results. Keys and passes are launch_bin_sort's (packed
-// when tile, Gaussian and the 31 bits that a positive depth can span fit), so the output
+// when tile, Gaussian and 32 depth bits fit), so the output
 // equals it.
 // ---------------------------------------------------------------------------------------
 __device__ __forceinline__ KeyLayout dev_layout(const uint64_t* __restrict__ E_dev, int64_t E_cap,
@@ -900,7 +915,6 @@ static Status sort_entries_dev(Ctx* c, const float* proj, const uint32_t* entry_
                                const uint64_t* E_dev, int64_t E_cap, const uint32_t* dr, uint32_t tiles_x,
                                uint32_t num_tiles, int tbits, int vbits, void* scratch, uint32_t* gauss_out,
                                uint32_t* ranges, uint32_t* overflow, const BatchTable* bt, int64_t n_view) {
-  const int max_passes = (tbits + 31 + 7) / 8;  // depths are positive floats: they span 31 bits at most
   const int64_t cap = std::max<int64_t>(E_cap, 1);
   const uint64_t tiles = sort_tiles(cap);
   // Carve the scratch (256-byte aligned pieces).
@@ -917,14 +931,14 @@ static Status sort_entries_dev(Ctx* c, const float* proj, const uint32_t* entry_
   const SortCtl ctl = carve_sort_ctl(carve(sort_ctl_bytes(cap)), cap);
   // One launch clears the tile ranges, the look-back words of the passes these keys can need,
   // and the histograms, tickets and abort word.
-  SPLAT_TRY(launch_zero3_u32(c, ranges, (size_t)num_tiles * 2, ctl.status, status_bytes(cap, max_passes) / 4, ctl.hist,
+  SPLAT_TRY(launch_zero3_u32(c, ranges, (size_t)num_tiles * 2, ctl.status, status_bytes(cap, max_passes(tbits)) / 4, ctl.hist,
                              kSortCounterWords));
   if (n > 0) {
     SPLAT_TRY(launch_chained(c, "emit_keys_dev_kernel", emit_keys_dev_kernel<kPacked>, emit_blocks(c, n), 256, 0,
                              reinterpret_cast<const float4*>(proj), entry_offset, n, tiles_x, dr, E_dev, E_cap,
                              tbits, vbits, b.ka, b.va, ctl.hist, overflow, bt, n_view));
   }
-  for (int pass = 0; pass < max_passes; pass++) {
+  for (int pass = 0; pass < max_passes(tbits); pass++) {
 #define SPLAT_PASS(S)                                                                                          \
   SPLAT_TRY((launch_pass<S>(c, radix_onesweep_dev_kernel<S, kPacked, W>, onesweep_smem<S, kPacked>(), tiles, b, \
                             E_dev, E_cap, dr, tbits, vbits, pass, ctl, tiles, overflow, gauss_out)))
@@ -948,7 +962,7 @@ Status launch_bin_sort_dev(Ctx* c, const float* proj, const uint32_t* entry_offs
   const uint32_t tiles_x = c->raster.tiles_x(width), tiles_y = c->raster.tiles_y(height);
   const uint32_t num_tiles = bt ? tiles_cap : tiles_x * tiles_y;
   const int tbits = bits_for(num_tiles), nbits = bits_for((uint64_t)std::max<int64_t>(n, 1));
-  const bool packed = tbits + 31 + nbits <= 64;
+  const bool packed = tbits + 32 + nbits <= 64;
   const int vbits = packed ? nbits : 0;
   n_view = std::max<int64_t>(n_view, 1);
 #define SPLAT_SORT(P, W)                                                                                              \
