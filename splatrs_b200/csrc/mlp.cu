@@ -21,6 +21,7 @@
 
 #include "common.cuh"
 #include "kernels.cuh"
+#include "pair.cuh"
 
 namespace splat {
 
@@ -418,12 +419,14 @@ constexpr int kTcRows = 128;
 constexpr uint32_t kTmemCols = 64;
 
 struct TcSmem {
-  alignas(1024) unsigned char ax[kTcRows * kIn * 2];    // A layer 1: [128][16]
-  alignas(1024) unsigned char ah[kTcRows * kHid * 2];   // A layers 2-3: [128][64]
-  alignas(1024) unsigned char bw1[kHid * kIn * 2];      // B layer 1: [64 out][16 in]
-  alignas(1024) unsigned char bw2[kHid * kHid * 2];     // B layer 2: [64 out][64 in]
-  alignas(1024) unsigned char bw3[16 * kHid * 2];       // B layer 3: [16 out (3 used)][64 in]
-  float b1[kHid], b2[kHid], b3[16];
+  // A operand: [128][16] of layer 1, then [128][64] of layers 2 and 3 (each written once the
+  // MMAs that read the one before have been waited for).
+  alignas(128) unsigned char a[kTcRows * kHid * 2];
+  alignas(128) unsigned char bw1[kHid * kIn * 2];   // B layer 1: [64 out][16 in], halved
+  alignas(128) unsigned char bw2[kHid * kHid * 2];  // B layer 2: [64 out][64 in], halved
+  alignas(128) unsigned char bw3[16 * kHid * 2];    // B layer 3: [16 out (3 used)][64 in]
+  alignas(16) float b1[kHid], b2[kHid];             // halved
+  float b3[16];
   alignas(8) uint64_t mbar;
   uint32_t tmem_base;
 };
@@ -475,36 +478,101 @@ __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence:
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void async_proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-// 16 consecutive accumulator columns of this thread's row.
-__device__ __forceinline__ void tmem_ld16(uint32_t addr, float v[16]) {
-  uint32_t r[16];
+// 16 consecutive accumulator columns of this thread's row: the load is issued, and
+// tmem_wait() makes the registers of every load issued before it valid.
+__device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t r[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
         "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(addr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+// (The registers pass through, so that no use of them moves ahead of the wait.)
+__device__ __forceinline__ void tmem_wait(uint32_t r[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                 "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+               :
+               : "memory");
+}
+__device__ __forceinline__ void tmem_read16(uint32_t addr, float v[16]) {
+  uint32_t r[16];
+  tmem_ld16(addr, r);
+  tmem_wait(r);
 #pragma unroll
   for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
 
-// Hidden layer epilogue: this thread's row of the accumulator at column col0, plus bias,
-// SiLU, rounded to BF16 into the A operand of the next layer.
-__device__ __forceinline__ void hidden_epilogue(TcSmem& s, uint32_t tmem_row, uint32_t col0, const float* bias,
-                                                int row) {
+// The hidden layers' weights and biases are laid out halved (exact: a power of two), so the
+// accumulators hold h = z / 2 and, with t = tanh(h), SiLU(z) = z (1 + t) / 2 = h + h t is one
+// tanh and one fused multiply-add.
+__device__ __forceinline__ f2 tanh_pair(f2 h) {
+  float lo, hi;
+  f2_split(h, lo, hi);
+  return f2_make(tanh_fast(lo), tanh_fast(hi));
+}
+__device__ __forceinline__ uint32_t pack2(f2 v) {
+  float lo, hi;
+  f2_split(v, lo, hi);
+  return pack2(lo, hi);
+}
+
+// Hidden layer epilogue: 64 accumulator columns from col0 of this thread's row, plus bias,
+// SiLU, rounded to BF16 into columns 0..63 of a K-major buffer of kdim columns. The next 16
+// columns are on their way while this 16 is worked on.
+__device__ __forceinline__ void silu_to(unsigned char* buf, int kdim, uint32_t tmem_row, uint32_t col0,
+                                        const float* bias, int row) {
+  uint32_t v[2][16];
+  tmem_ld16(tmem_row + col0, v[0]);
 #pragma unroll
   for (int c = 0; c < kHid; c += 16) {
-    float v[16];
-    tmem_ld16(tmem_row + col0 + c, v);
+    uint32_t(&z)[16] = v[(c >> 4) & 1];
+    tmem_wait(z);
+    if (c + 16 < kHid) tmem_ld16(tmem_row + col0 + c + 16, v[((c >> 4) + 1) & 1]);
 #pragma unroll
-    for (int h = 0; h < 16; h += 8) {  // one 16-byte core-matrix row per store
+    for (int q = 0; q < 16; q += 8) {  // one 16-byte core-matrix row per store
       uint32_t w[4];
 #pragma unroll
-      for (int i = 0; i < 4; i++)
-        w[i] = pack2(silu(v[h + 2 * i] + bias[c + h + 2 * i]), silu(v[h + 2 * i + 1] + bias[c + h + 2 * i + 1]));
-      *reinterpret_cast<uint4*>(s.ah + core_off(row, c + h, kHid)) = make_uint4(w[0], w[1], w[2], w[3]);
+      for (int i = 0; i < 8; i += 4) {
+        const float4 b = *reinterpret_cast<const float4*>(bias + c + q + i);
+        const f2 h0 = f2_add(f2_make(__uint_as_float(z[q + i]), __uint_as_float(z[q + i + 1])), f2_make(b.x, b.y));
+        const f2 h1 = f2_add(f2_make(__uint_as_float(z[q + i + 2]), __uint_as_float(z[q + i + 3])), f2_make(b.z, b.w));
+        w[i / 2] = pack2(f2_fma(h0, tanh_pair(h0), h0));
+        w[i / 2 + 1] = pack2(f2_fma(h1, tanh_pair(h1), h1));
+      }
+      *reinterpret_cast<uint4*>(buf + core_off(row, c + q, kdim)) = make_uint4(w[0], w[1], w[2], w[3]);
     }
   }
+}
+
+// `rows` x `cols` weights at w, element (r, k) at w[r * rs + k * ks] times mul, rounded to BF16
+// into a K-major operand; rows past `live` and columns past `klive` are zero. A thread fills
+// whole 16-byte core-matrix rows; kRowsFast: neighbouring threads take neighbouring rows
+// (weights contiguous along r), else neighbouring 8-column pieces.
+template <bool kRowsFast>
+__device__ __forceinline__ void lay_out(unsigned char* buf, const float* __restrict__ w, int rows, int cols, int rs,
+                                        int ks, int live, int klive, float mul) {
+  for (int i = threadIdx.x; i < rows * cols / 8; i += kTcRows) {
+    const int r = kRowsFast ? i % rows : i / (cols / 8), k = 8 * (kRowsFast ? i / rows : i % (cols / 8));
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) v[j] = r < live && k + j < klive ? mul * w[r * rs + (k + j) * ks] : 0.0f;
+    *reinterpret_cast<uint4*>(buf + core_off(r, k, cols)) =
+        make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
+  }
+}
+// The forward's three weight operands and its biases.
+__device__ __forceinline__ void lay_out_forward(const float* __restrict__ th, unsigned char* bw1, unsigned char* bw2,
+                                                unsigned char* bw3, float* b1, float* b2, float* b3) {
+  lay_out<true>(bw1, th + kW1, kHid, kIn, 1, kHid, kHid, kIn, 0.5f);
+  lay_out<true>(bw2, th + kW2, kHid, kHid, 1, kHid, kHid, kHid, 0.5f);
+  lay_out<true>(bw3, th + kW3, 16, kHid, 1, kOut, kOut, kHid, 1.0f);
+  const int tid = threadIdx.x;
+  if (tid < kHid) {
+    b1[tid] = 0.5f * th[kB1 + tid];
+    b2[tid] = 0.5f * th[kB2 + tid];
+  }
+  if (tid < 16) b3[tid] = tid < kOut ? th[kB3 + tid] : 0.0f;
 }
 
 // A 128-row tile of feature rows (512 float4, contiguous) into registers, coalesced:
@@ -521,12 +589,16 @@ __device__ __forceinline__ void load_tile(const float* __restrict__ x, int64_t t
 
 // Persistent: a CTA lays the weights out once and loops over 128-row tiles with stride
 // gridDim.x, loading the next tile's rows into registers while this tile's MMAs run.
+// 128 hyperbolic tangents per row bind the special-function unit: 14 us of the 30.0 us that
+// 500,000 rows take (37.4 us with 33 KB of shared memory, six CTAs on an SM instead of seven,
+// a multiply and an add more per activation, and weights laid out one element at a time).
+// The rest is the chain of three MMAs and epilogues per tile and the last round of tiles.
 __global__ void __launch_bounds__(kTcRows) mlp_forward_tc_kernel(const float* __restrict__ x, int64_t n,
                                                                   const float* __restrict__ th,
                                                                   float* __restrict__ prob,
                                                                   volatile uint32_t* __restrict__ err) {
   extern __shared__ unsigned char tc_raw[];
-  TcSmem& s = *reinterpret_cast<TcSmem*>((reinterpret_cast<uintptr_t>(tc_raw) + 1023) & ~(uintptr_t)1023);
+  TcSmem& s = *reinterpret_cast<TcSmem*>((reinterpret_cast<uintptr_t>(tc_raw) + 127) & ~(uintptr_t)127);
   const int tid = threadIdx.x, warp = tid >> 5;
   const int64_t tiles = (n + kTcRows - 1) / kTcRows;
   if (tid == 0) {
@@ -540,25 +612,10 @@ __global__ void __launch_bounds__(kTcRows) mlp_forward_tc_kernel(const float* __
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  // Weights, rounded to BF16, in the K-major operand layouts.
-  for (int i = tid; i < kIn * kHid; i += kTcRows) {
-    const int in = i / kHid, out = i % kHid;
-    *reinterpret_cast<bf*>(s.bw1 + core_off(out, in, kIn)) = __float2bfloat16_rn(th[kW1 + i]);
-  }
-  for (int i = tid; i < kHid * kHid; i += kTcRows) {
-    const int in = i / kHid, out = i % kHid;
-    *reinterpret_cast<bf*>(s.bw2 + core_off(out, in, kHid)) = __float2bfloat16_rn(th[kW2 + i]);
-  }
-  for (int i = tid; i < 16 * kHid; i += kTcRows) {
-    const int out = i / kHid, in = i % kHid;
-    const float w = out < kOut ? th[kW3 + in * kOut + out] : 0.0f;
-    *reinterpret_cast<bf*>(s.bw3 + core_off(out, in, kHid)) = __float2bfloat16_rn(w);
-  }
-  if (tid < kHid) {
-    s.b1[tid] = th[kB1 + tid];
-    s.b2[tid] = th[kB2 + tid];
-  }
-  if (tid < 16) s.b3[tid] = tid < kOut ? th[kB3 + tid] : 0.0f;
+  float4 xr[4];
+  int64_t tile = blockIdx.x;
+  if (tile < tiles) load_tile(x, tile, n, xr);
+  lay_out_forward(th, s.bw1, s.bw2, s.bw3, s.b1, s.b2, s.b3);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -566,15 +623,12 @@ __global__ void __launch_bounds__(kTcRows) mlp_forward_tc_kernel(const float* __
   const uint32_t tmem_row = tmem + ((uint32_t)(32 * warp) << 16);
   bool ok = true;
   uint32_t phase = 0;
-  float4 xr[4];
-  int64_t tile = blockIdx.x;
-  if (tile < tiles) load_tile(x, tile, n, xr);
   for (; tile < tiles; tile += gridDim.x) {
     const int64_t row_g = tile * kTcRows + tid;
 #pragma unroll
     for (int q = 0; q < 4; q++) {
       const int f = tid + kTcRows * q;  // row f / 4, columns 4 (f % 4) .. + 3
-      *reinterpret_cast<uint2*>(s.ax + core_off(f >> 2, (f & 3) * 4, kIn)) =
+      *reinterpret_cast<uint2*>(s.a + core_off(f >> 2, (f & 3) * 4, kIn)) =
           make_uint2(pack2(xr[q].x, xr[q].y), pack2(xr[q].z, xr[q].w));
     }
     async_proxy_fence();
@@ -583,7 +637,7 @@ __global__ void __launch_bounds__(kTcRows) mlp_forward_tc_kernel(const float* __
     tc_fence_after();
     // Layer 1: [128 x 16] x [16 x 64] into columns 0-63.
     if (tid == 0) {
-      tc_mma(tmem, smem_desc(s.ax, 256), smem_desc(s.bw1, 256), idesc_bf16(kHid), 0u);
+      tc_mma(tmem, smem_desc(s.a, 256), smem_desc(s.bw1, 256), idesc_bf16(kHid), 0u);
       tc_commit(&s.mbar);
     }
     if (tile + gridDim.x < tiles) load_tile(x, tile + gridDim.x, n, xr);
@@ -591,7 +645,7 @@ __global__ void __launch_bounds__(kTcRows) mlp_forward_tc_kernel(const float* __
     if (!ok) break;
     phase ^= 1u;
     tc_fence_after();
-    hidden_epilogue(s, tmem_row, 0, s.b1, tid);
+    silu_to(s.a, kHid, tmem_row, 0, s.b1, tid);
     async_proxy_fence();
     tc_fence_before();
     __syncthreads();
@@ -600,7 +654,7 @@ __global__ void __launch_bounds__(kTcRows) mlp_forward_tc_kernel(const float* __
     if (tid == 0) {
 #pragma unroll
       for (int k = 0; k < 4; k++)
-        tc_mma(tmem, smem_desc(s.ah + 256 * k, 1024), smem_desc(s.bw2 + 256 * k, 1024), idesc_bf16(kHid),
+        tc_mma(tmem, smem_desc(s.a + 256 * k, 1024), smem_desc(s.bw2 + 256 * k, 1024), idesc_bf16(kHid),
                k > 0 ? 1u : 0u);
       tc_commit(&s.mbar);
     }
@@ -608,7 +662,7 @@ __global__ void __launch_bounds__(kTcRows) mlp_forward_tc_kernel(const float* __
     if (!ok) break;
     phase ^= 1u;
     tc_fence_after();
-    hidden_epilogue(s, tmem_row, 0, s.b2, tid);
+    silu_to(s.a, kHid, tmem_row, 0, s.b2, tid);
     async_proxy_fence();
     tc_fence_before();
     __syncthreads();
@@ -617,7 +671,7 @@ __global__ void __launch_bounds__(kTcRows) mlp_forward_tc_kernel(const float* __
     if (tid == 0) {
 #pragma unroll
       for (int k = 0; k < 4; k++)
-        tc_mma(tmem, smem_desc(s.ah + 256 * k, 1024), smem_desc(s.bw3 + 256 * k, 1024), idesc_bf16(16),
+        tc_mma(tmem, smem_desc(s.a + 256 * k, 1024), smem_desc(s.bw3 + 256 * k, 1024), idesc_bf16(16),
                k > 0 ? 1u : 0u);
       tc_commit(&s.mbar);
     }
@@ -626,7 +680,7 @@ __global__ void __launch_bounds__(kTcRows) mlp_forward_tc_kernel(const float* __
     phase ^= 1u;
     tc_fence_after();
     float v[16];
-    tmem_ld16(tmem_row, v);
+    tmem_read16(tmem_row, v);
     const float z0 = v[0] + s.b3[0], z1 = v[1] + s.b3[1], z2 = v[2] + s.b3[2];
     const float m = fmaxf(z0, fmaxf(z1, z2));
     const float e0 = __expf(z0 - m), e1 = __expf(z1 - m), e2 = __expf(z2 - m);
@@ -649,39 +703,47 @@ __global__ void __launch_bounds__(kTcRows) mlp_forward_tc_kernel(const float* __
   }
 }
 // ---------------------------------------------------------------------------------------
-// The gradient on tcgen05: the forward of a 128-row tile as above with its layer outputs
-// z1, z2, z3 kept in tensor memory, then
+// The gradient on tcgen05: the forward of a 128-row tile as above, then
 //   dh2 = dz3 W3^T and dh1 = dz2 W2^T     (M = the tile's rows, K-major operands), and
-//   [dW2^T ; dW1^T] = [dz2 | dz1]^T [h1 | x]   and   dW3^T = [. | dz3 | .]^T h2,
+//   [dW2^T ; dW1^T] = [dz2 | dz1]^T [h1 | x]   and   [dW3 ; .] = [h2 | .]^T dz3,
 // the weight gradients as two M = 128 products over the tile's rows (K), which read the
 // same shared-memory buffers as MN-major operands: a buffer laid out K-major for one
 // product is, core matrix for core matrix, the MN-major operand of the transposed one.
-// dW2^T and dW1^T are the diagonal blocks of one 128 x 80 product; dW3^T is rows 64-66 of a
-// 128 x 64 one whose A is the dz buffer while dz3 sits in its columns 64-79. Both
-// accumulate in tensor memory over all of the CTA's tiles and reach global memory once.
-// Bias gradients (unrounded dz) go through shared memory. Rounding points are those of the
-// mma.sync kernel and the oracle's bf16 mode.
+// dW2^T and dW1^T are the diagonal blocks of one 128 x 80 product. dW3 is rows 0-63 of a
+// 128 x 16 one: h2 has 64 columns, so the A operand's core matrices 8-15 of a row group are
+// those of the group after it (past the last group, the dz buffer's first), and rows 64-127
+// of the product are never read. Both accumulate in tensor memory over all of the CTA's
+// tiles and reach global memory once. Bias gradients (unrounded dz) are reduced across the
+// lanes of each warp and kept in registers. Rounding points are those of the mma.sync kernel
+// and the oracle's bf16 mode.
+//
+// A tile is seven dependent steps of MMA, wait and epilogue: latency, not a rate, bounds it,
+// so the point is to have two CTAs on an SM. That takes half of the tensor memory (224
+// columns of 512: z1 is multiplied out again, beside dh1, instead of being kept, and z3
+// shares its columns with dh2 and dh1) and no staging tile for the bias gradients. 65,536
+// rows: 43.0 us with one CTA (368 columns, a 33 KB staging tile), 26.1 us with two.
 // ---------------------------------------------------------------------------------------
-constexpr uint32_t kGradTmemCols = 512;
-constexpr uint32_t kZ1 = 0, kZ2 = 64, kZ3 = 128, kDH = 160, kAcc3 = 224, kAccW = 288;
+constexpr uint32_t kGradTmemCols = 256;
+constexpr uint32_t kZ = 0, kDH = 64, kAcc3 = 128, kAccW = 144;
 constexpr int kXH = 80;   // columns of the [h1 | x] buffer
 constexpr int kDZ = 128;  // columns of the [dz2 | dz1] buffer (dz3 in 64-79 before dz1)
 
 struct TcGradSmem {
-  alignas(1024) unsigned char xh[kTcRows * kXH * 2];
-  alignas(1024) unsigned char h2[kTcRows * kHid * 2];
-  alignas(1024) unsigned char dz[kTcRows * kDZ * 2];
-  alignas(1024) unsigned char w1t[kHid * kIn * 2];   // B of layer 1: [out][in], K = in
-  alignas(1024) unsigned char w2t[kHid * kHid * 2];  // B of layer 2: [out][in]
-  alignas(1024) unsigned char w3t[16 * kHid * 2];    // B of layer 3: [out (16)][in]
-  alignas(1024) unsigned char w2n[kHid * kHid * 2];  // B of dh1 = dz2 W2^T: [in][out], K = out
-  alignas(1024) unsigned char w3n[kHid * 16 * 2];    // B of dh2 = dz3 W3^T: [in][out (16)]
-  float b1[kHid], b2[kHid], b3[16];
+  alignas(128) unsigned char xh[kTcRows * kXH * 2];
+  alignas(128) unsigned char h2[kTcRows * kHid * 2];
+  alignas(128) unsigned char dz[kTcRows * kDZ * 2];   // right after h2: see dW3
+  alignas(128) unsigned char w1t[kHid * kIn * 2];     // B of layer 1: [out][in], K = in, halved
+  alignas(128) unsigned char w2t[kHid * kHid * 2];    // B of layer 2: [out][in], halved
+  alignas(128) unsigned char w3t[16 * kHid * 2];      // B of layer 3: [out (16)][in]
+  alignas(128) unsigned char w2n[kHid * kHid * 2];    // B of dh1 = dz2 W2^T: [in][out], K = out
+  alignas(128) unsigned char w3n[kHid * 16 * 2];      // B of dh2 = dz3 W3^T: [in][out (16)]
+  alignas(16) float b1[kHid], b2[kHid];               // halved
+  float b3[16];
   float gb[kHid + kHid + 16];  // bias gradients: b1, b2, b3
-  float f[kTcRows][kHid + 1];  // a tile's unrounded dz2 or dz1, for the column sums of the bias gradients
   alignas(8) uint64_t mbar;
   uint32_t tmem_base;
 };
+static_assert(offsetof(TcGradSmem, dz) == offsetof(TcGradSmem, h2) + kTcRows * kHid * 2, "dz follows h2");
 
 __host__ __device__ constexpr uint32_t idesc_bf16_major(uint32_t n, uint32_t a_mn, uint32_t b_mn) {
   return idesc_bf16(n) | (a_mn << 15) | (b_mn << 16);
@@ -693,57 +755,54 @@ __device__ __forceinline__ uint64_t smem_desc_lbo(const void* p, uint32_t lbo, u
          ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
 
-// Reads 64 accumulator columns from col0 of this thread's row, adds the bias and writes
-// SiLU of the sum, rounded to BF16, to columns 0..63 of a K-major buffer of kdim columns.
-__device__ __forceinline__ void silu_to(unsigned char* buf, int kdim, uint32_t tmem_row, uint32_t col0,
-                                        const float* bias, int row) {
+// Sum over the warp's 32 rows of each of 16 columns: lane l is left with column l % 16.
+__device__ __forceinline__ float column_sum16(float d[16], int lane) {
 #pragma unroll
-  for (int c = 0; c < kHid; c += 16) {
-    float v[16];
-    tmem_ld16(tmem_row + col0 + c, v);
+  for (int o = 8; o > 0; o >>= 1) {
+    const bool hi = lane & o;
 #pragma unroll
-    for (int h = 0; h < 16; h += 8) {
-      uint32_t w[4];
-#pragma unroll
-      for (int i = 0; i < 4; i++)
-        w[i] = pack2(silu(v[h + 2 * i] + bias[c + h + 2 * i]), silu(v[h + 2 * i + 1] + bias[c + h + 2 * i + 1]));
-      *reinterpret_cast<uint4*>(buf + core_off(row, c + h, kdim)) = make_uint4(w[0], w[1], w[2], w[3]);
+    for (int i = 0; i < o; i++) {
+      const float give = hi ? d[i] : d[i + o], keep = hi ? d[i + o] : d[i];
+      d[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
     }
   }
+  return d[0] + __shfl_xor_sync(0xffffffffu, d[0], 16);
 }
 
-// dz = dh * SiLU'(z + bias) for 64 columns (dh at dh_col, z at z_col of this thread's row),
-// rounded to BF16 into columns col_out.. of the dz buffer; the unrounded dz into row `row`
-// of the staging tile f (a row past the batch has dz = 0: its weight is 0).
-__device__ __forceinline__ void dz_to(TcGradSmem& s, uint32_t tmem_row, uint32_t dh_col, uint32_t z_col,
-                                      const float* bias, int col_out, int row) {
+// dz = dh * SiLU'(z) for 64 columns (dh at kDH, h = z / 2 without its bias at kZ of this
+// thread's row), rounded to BF16 into columns col_out.. of the dz buffer; the unrounded dz's
+// column sums over the warp's rows are added to gacc (lane l: columns l % 16 + 16 q; a row
+// past the batch has dz = 0: its weight is 0). With t = tanh(h) and u = (1 + t) / 2,
+// SiLU'(z) = u + u (h - h t).
+__device__ __forceinline__ void dz_to(TcGradSmem& s, uint32_t tmem_row, const float* bias, int col_out, int row,
+                                      float gacc[4]) {
+  const f2 half = f2_splat(0.5f);
 #pragma unroll
   for (int c = 0; c < kHid; c += 16) {
-    float d[16], z[16];
-    tmem_ld16(tmem_row + dh_col + c, d);
-    tmem_ld16(tmem_row + z_col + c, z);
+    uint32_t rd[16], rz[16];
+    float d[16];
+    tmem_ld16(tmem_row + kDH + c, rd);
+    tmem_ld16(tmem_row + kZ + c, rz);
+    tmem_wait(rd);
+    tmem_wait(rz);
 #pragma unroll
-    for (int i = 0; i < 16; i++) d[i] *= silu_grad(z[i] + bias[c + i]);
-#pragma unroll
-    for (int h = 0; h < 16; h += 8) {
-      uint32_t w[4];
-#pragma unroll
-      for (int i = 0; i < 4; i++) w[i] = pack2(d[h + 2 * i], d[h + 2 * i + 1]);
-      *reinterpret_cast<uint4*>(s.dz + core_off(row, col_out + c + h, kDZ)) = make_uint4(w[0], w[1], w[2], w[3]);
+    for (int i = 0; i < 16; i += 2) {
+      const float2 b = *reinterpret_cast<const float2*>(bias + c + i);
+      const f2 h = f2_add(f2_make(__uint_as_float(rz[i]), __uint_as_float(rz[i + 1])), f2_make(b.x, b.y));
+      const f2 t = tanh_pair(h), u = f2_fma(half, t, half);
+      float h0, h1, t0, t1;
+      f2_split(h, h0, h1);
+      f2_split(t, t0, t1);
+      const f2 g = f2_fma(u, f2_make(__fmaf_rn(-h0, t0, h0), __fmaf_rn(-h1, t1, h1)), u);
+      f2_split(f2_mul(f2_make(__uint_as_float(rd[i]), __uint_as_float(rd[i + 1])), g), d[i], d[i + 1]);
     }
 #pragma unroll
-    for (int i = 0; i < 16; i++) s.f[row][c + i] = d[i];
+    for (int q = 0; q < 16; q += 8)
+      *reinterpret_cast<uint4*>(s.dz + core_off(row, col_out + c + q, kDZ)) =
+          make_uint4(pack2(d[q], d[q + 1]), pack2(d[q + 2], d[q + 3]), pack2(d[q + 4], d[q + 5]),
+                     pack2(d[q + 6], d[q + 7]));
+    gacc[c >> 4] += column_sum16(d, threadIdx.x & 31);
   }
-}
-
-// This thread's share of the staging tile's column sums: column tid % 64 over half of the
-// rows (conflict-free: the tile's rows are 65 floats apart).
-__device__ __forceinline__ float column_half_sum(const TcGradSmem& s, int tid) {
-  const int col = tid & (kHid - 1), r0 = (tid >> 6) * (kTcRows / 2);
-  float acc = 0.0f;
-#pragma unroll 8
-  for (int r = 0; r < kTcRows / 2; r++) acc += s.f[r0 + r][col];
-  return acc;
 }
 
 __global__ void __launch_bounds__(kTcRows) mlp_grad_tc_kernel(const float* __restrict__ x,
@@ -752,7 +811,7 @@ __global__ void __launch_bounds__(kTcRows) mlp_grad_tc_kernel(const float* __res
                                                                const float* __restrict__ th, float* __restrict__ grad,
                                                                volatile uint32_t* __restrict__ err) {
   extern __shared__ unsigned char tc_raw[];
-  TcGradSmem& s = *reinterpret_cast<TcGradSmem*>((reinterpret_cast<uintptr_t>(tc_raw) + 1023) & ~(uintptr_t)1023);
+  TcGradSmem& s = *reinterpret_cast<TcGradSmem*>((reinterpret_cast<uintptr_t>(tc_raw) + 127) & ~(uintptr_t)127);
   const int tid = threadIdx.x, warp = tid >> 5;
   const int64_t tiles = (n + kTcRows - 1) / kTcRows;
   if (tid == 0) {
@@ -766,27 +825,12 @@ __global__ void __launch_bounds__(kTcRows) mlp_grad_tc_kernel(const float* __res
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  for (int i = tid; i < kIn * kHid; i += kTcRows) {
-    const int in = i / kHid, out = i % kHid;
-    *reinterpret_cast<bf*>(s.w1t + core_off(out, in, kIn)) = __float2bfloat16_rn(th[kW1 + i]);
-  }
-  for (int i = tid; i < kHid * kHid; i += kTcRows) {
-    const int in = i / kHid, out = i % kHid;
-    const bf v = __float2bfloat16_rn(th[kW2 + i]);
-    *reinterpret_cast<bf*>(s.w2t + core_off(out, in, kHid)) = v;
-    *reinterpret_cast<bf*>(s.w2n + core_off(in, out, kHid)) = v;
-  }
-  for (int i = tid; i < 16 * kHid; i += kTcRows) {
-    const int out = i / kHid, in = i % kHid;
-    const bf v = __float2bfloat16_rn(out < kOut ? th[kW3 + in * kOut + out] : 0.0f);
-    *reinterpret_cast<bf*>(s.w3t + core_off(out, in, kHid)) = v;
-    *reinterpret_cast<bf*>(s.w3n + core_off(in, out, 16)) = v;
-  }
-  if (tid < kHid) {
-    s.b1[tid] = th[kB1 + tid];
-    s.b2[tid] = th[kB2 + tid];
-  }
-  if (tid < 16) s.b3[tid] = tid < kOut ? th[kB3 + tid] : 0.0f;
+  float4 xr[4];
+  int64_t tile = blockIdx.x;
+  if (tile < tiles) load_tile(x, tile, n, xr);
+  lay_out_forward(th, s.w1t, s.w2t, s.w3t, s.b1, s.b2, s.b3);
+  lay_out<false>(s.w2n, th + kW2, kHid, kHid, kHid, 1, kHid, kHid, 1.0f);
+  lay_out<false>(s.w3n, th + kW3, kHid, 16, kOut, 1, kHid, kOut, 1.0f);
   for (int i = tid; i < kHid + kHid + 16; i += kTcRows) s.gb[i] = 0.0f;
   for (int i = tid; i < kTcRows * kDZ / 8; i += kTcRows) reinterpret_cast<uint4*>(s.dz)[i] = make_uint4(0, 0, 0, 0);
   tc_fence_before();
@@ -796,10 +840,7 @@ __global__ void __launch_bounds__(kTcRows) mlp_grad_tc_kernel(const float* __res
   const uint32_t tmem_row = tmem + ((uint32_t)(32 * warp) << 16);
   bool ok = true, first = true;
   uint32_t phase = 0;
-  float gacc1 = 0.0f, gacc2 = 0.0f;  // this thread's share of the b1 and b2 gradients
-  float4 xr[4];
-  int64_t tile = blockIdx.x;
-  if (tile < tiles) load_tile(x, tile, n, xr);
+  float gacc1[4] = {}, gacc2[4] = {}, gacc3[kOut] = {};  // this thread's share of the bias gradients
   // One wait for the MMAs committed by thread 0; the whole block agrees on the outcome.
 #define SPLAT_TC_WAIT()                                          \
   do {                                                           \
@@ -828,35 +869,35 @@ __global__ void __launch_bounds__(kTcRows) mlp_grad_tc_kernel(const float* __res
     }
     SPLAT_TC_HANDOFF();
     if (tid == 0) {  // z1 = x W1
-      tc_mma(tmem + kZ1, smem_desc_lbo(s.xh + 8 * 128, 128, kXH / 8 * 128), smem_desc(s.w1t, 256), idesc_bf16(kHid),
+      tc_mma(tmem + kZ, smem_desc_lbo(s.xh + 8 * 128, 128, kXH / 8 * 128), smem_desc(s.w1t, 256), idesc_bf16(kHid),
              0u);
       tc_commit(&s.mbar);
     }
     if (tile + gridDim.x < tiles) load_tile(x, tile + gridDim.x, n, xr);
     SPLAT_TC_WAIT();
-    silu_to(s.xh, kXH, tmem_row, kZ1, s.b1, tid);  // h1 into columns 0-63
+    silu_to(s.xh, kXH, tmem_row, kZ, s.b1, tid);  // h1 into columns 0-63
     SPLAT_TC_HANDOFF();
     if (tid == 0) {  // z2 = h1 W2
 #pragma unroll
       for (int k = 0; k < 4; k++)
-        tc_mma(tmem + kZ2, smem_desc_lbo(s.xh + 256 * k, 128, kXH / 8 * 128), smem_desc(s.w2t + 256 * k, 1024),
+        tc_mma(tmem + kZ, smem_desc_lbo(s.xh + 256 * k, 128, kXH / 8 * 128), smem_desc(s.w2t + 256 * k, 1024),
                idesc_bf16(kHid), k > 0 ? 1u : 0u);
       tc_commit(&s.mbar);
     }
     SPLAT_TC_WAIT();
-    silu_to(s.h2, kHid, tmem_row, kZ2, s.b2, tid);
+    silu_to(s.h2, kHid, tmem_row, kZ, s.b2, tid);
     SPLAT_TC_HANDOFF();
     if (tid == 0) {  // z3 = h2 W3
 #pragma unroll
       for (int k = 0; k < 4; k++)
-        tc_mma(tmem + kZ3, smem_desc(s.h2 + 256 * k, 1024), smem_desc(s.w3t + 256 * k, 1024), idesc_bf16(16),
+        tc_mma(tmem + kDH, smem_desc(s.h2 + 256 * k, 1024), smem_desc(s.w3t + 256 * k, 1024), idesc_bf16(16),
                k > 0 ? 1u : 0u);
       tc_commit(&s.mbar);
     }
     SPLAT_TC_WAIT();
     {  // softmax and dz3 = (p - onehot(y)) w scale, into dz columns 64-79
       float v[16];
-      tmem_ld16(tmem_row + kZ3, v);
+      tmem_read16(tmem_row + kDH, v);
       const float z0 = v[0] + s.b3[0], z1 = v[1] + s.b3[1], z2 = v[2] + s.b3[2];
       const float m = fmaxf(z0, fmaxf(z1, z2));
       const float e0 = __expf(z0 - m), e1 = __expf(z1 - m), e2 = __expf(z2 - m);
@@ -866,45 +907,37 @@ __global__ void __launch_bounds__(kTcRows) mlp_grad_tc_kernel(const float* __res
       const float d2 = (e2 * inv - (yl == 2 ? 1.0f : 0.0f)) * wl;
       *reinterpret_cast<uint4*>(s.dz + core_off(tid, kHid, kDZ)) = make_uint4(pack2(d0, d1), pack2(d2, 0.0f), 0u, 0u);
       *reinterpret_cast<uint4*>(s.dz + core_off(tid, kHid + 8, kDZ)) = make_uint4(0u, 0u, 0u, 0u);
-      float r0 = d0, r1 = d1, r2 = d2;  // b3 gradient: the warp's sums, one atomic each
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        r0 += __shfl_xor_sync(0xffffffffu, r0, o);
-        r1 += __shfl_xor_sync(0xffffffffu, r1, o);
-        r2 += __shfl_xor_sync(0xffffffffu, r2, o);
-      }
-      if ((tid & 31) == 0) {
-        atomicAdd(&s.gb[2 * kHid], r0);
-        atomicAdd(&s.gb[2 * kHid + 1], r1);
-        atomicAdd(&s.gb[2 * kHid + 2], r2);
-      }
+      gacc3[0] += d0;
+      gacc3[1] += d1;
+      gacc3[2] += d2;
     }
     SPLAT_TC_HANDOFF();
     if (tid == 0) {
       // dh2 = dz3 W3^T (K = 16 outputs, 3 used)
       tc_mma(tmem + kDH, smem_desc_lbo(s.dz + 8 * 128, 128, kDZ / 8 * 128), smem_desc(s.w3n, 256), idesc_bf16(kHid),
              0u);
-      // dW3^T += (dz columns)^T h2 over the tile's rows: A MN-major (M = 128 columns), B MN-major (N = 64)
+      // dW3 += h2^T dz3 over the tile's rows: A MN-major (M = 128 columns, 64 of h2's), B MN-major (N = 16)
 #pragma unroll
       for (int k = 0; k < kTcRows / 16; k++)
-        tc_mma(tmem + kAcc3, smem_desc_lbo(s.dz + 2 * k * (kDZ / 8 * 128), kDZ / 8 * 128, 128),
-               smem_desc_lbo(s.h2 + 2 * k * 1024, 1024, 128), idesc_bf16_major(kHid, 1u, 1u),
-               (first && k == 0) ? 0u : 1u);
+        tc_mma(tmem + kAcc3, smem_desc_lbo(s.h2 + 2 * k * 1024, 1024, 128),
+               smem_desc_lbo(s.dz + 8 * 128 + 2 * k * (kDZ / 8 * 128), kDZ / 8 * 128, 128),
+               idesc_bf16_major(16, 1u, 1u), (first && k == 0) ? 0u : 1u);
       tc_commit(&s.mbar);
     }
     SPLAT_TC_WAIT();
-    dz_to(s, tmem_row, kDH, kZ2, s.b2, 0, tid);  // dz2 into columns 0-63
+    dz_to(s, tmem_row, s.b2, 0, tid, gacc2);  // dz2 into columns 0-63
     SPLAT_TC_HANDOFF();
-    if (tid == 0) {  // dh1 = dz2 W2^T
+    if (tid == 0) {  // dh1 = dz2 W2^T, and z1 = x W1 once more
 #pragma unroll
       for (int k = 0; k < 4; k++)
         tc_mma(tmem + kDH, smem_desc_lbo(s.dz + 256 * k, 128, kDZ / 8 * 128), smem_desc(s.w2n + 256 * k, 1024),
                idesc_bf16(kHid), k > 0 ? 1u : 0u);
+      tc_mma(tmem + kZ, smem_desc_lbo(s.xh + 8 * 128, 128, kXH / 8 * 128), smem_desc(s.w1t, 256), idesc_bf16(kHid),
+             0u);
       tc_commit(&s.mbar);
     }
-    gacc2 += column_half_sum(s, tid);  // while the MMAs run
     SPLAT_TC_WAIT();
-    dz_to(s, tmem_row, kDH, kZ1, s.b1, kHid, tid);  // dz1 into columns 64-127
+    dz_to(s, tmem_row, s.b1, kHid, tid, gacc1);  // dz1 into columns 64-127
     SPLAT_TC_HANDOFF();
     if (tid == 0) {  // [dW2^T ; dW1^T] += [dz2 | dz1]^T [h1 | x]
 #pragma unroll
@@ -914,38 +947,45 @@ __global__ void __launch_bounds__(kTcRows) mlp_grad_tc_kernel(const float* __res
                (first && k == 0) ? 0u : 1u);
       tc_commit(&s.mbar);
     }
-    gacc1 += column_half_sum(s, tid);
     SPLAT_TC_WAIT();  // the buffers are free for the next tile
     first = false;
   }
   if (!first) {  // this CTA's accumulated weight gradients, once
-    if (warp == 2) {  // dW3^T rows 64-66: lanes 0-2
+    if (warp < 2) {  // dW3 rows 0-63, columns 0-2
+      float v[16];
+      tmem_read16(tmem_row + kAcc3, v);
 #pragma unroll
-      for (int c = 0; c < kHid; c += 16) {
-        float v[16];
-        tmem_ld16(tmem_row + kAcc3 + c, v);
-        const int out = tid - 2 * 32;
-        if (out < kOut)
-#pragma unroll
-          for (int i = 0; i < 16; i++) atomicAdd(&grad[kW3 + (c + i) * kOut + out], v[i]);
-      }
+      for (int o = 0; o < kOut; o++) atomicAdd(&grad[kW3 + tid * kOut + o], v[o]);
     }
     if (warp < 2) {  // dW2^T rows 0-63, columns 0-63
 #pragma unroll
       for (int c = 0; c < kHid; c += 16) {
         float v[16];
-        tmem_ld16(tmem_row + kAccW + c, v);
+        tmem_read16(tmem_row + kAccW + c, v);
 #pragma unroll
         for (int i = 0; i < 16; i++) atomicAdd(&grad[kW2 + (c + i) * kHid + tid], v[i]);
       }
     } else {  // dW1^T rows 64-127, columns 64-79
       float v[16];
-      tmem_ld16(tmem_row + kAccW + kHid, v);
+      tmem_read16(tmem_row + kAccW + kHid, v);
 #pragma unroll
       for (int i = 0; i < 16; i++) atomicAdd(&grad[kW1 + i * kHid + (tid - kHid)], v[i]);
     }
-    atomicAdd(&s.gb[tid & (kHid - 1)], gacc1);
-    atomicAdd(&s.gb[kHid + (tid & (kHid - 1))], gacc2);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int k = 0; k < kOut; k++) gacc3[k] += __shfl_xor_sync(0xffffffffu, gacc3[k], o);
+    const int lane = tid & 31;
+    if (lane < 16) {
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        atomicAdd(&s.gb[16 * q + lane], gacc1[q]);
+        atomicAdd(&s.gb[kHid + 16 * q + lane], gacc2[q]);
+      }
+    }
+    if (lane == 0)
+#pragma unroll
+      for (int k = 0; k < kOut; k++) atomicAdd(&s.gb[2 * kHid + k], gacc3[k]);
     __syncthreads();
     for (int i = tid; i < kHid; i += kTcRows) {
       atomicAdd(&grad[kB1 + i], s.gb[i]);
@@ -973,7 +1013,7 @@ int mlp_num_params() { return kParams; }
 
 Status launch_mlp_forward_tc(Ctx* c, const float* x, int64_t n, const float* theta, float* prob, uint32_t* err) {
   if (n == 0) return Status::ok();
-  const size_t smem = sizeof(TcSmem) + 1024;
+  const size_t smem = sizeof(TcSmem) + 128;
   SPLAT_CUDA(cudaFuncSetAttribute(mlp_forward_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int dev = 0, sms = 0, smem_sm = 0, smem_rsv = 0;
   SPLAT_CUDA(cudaGetDevice(&dev));
@@ -1023,13 +1063,13 @@ Status launch_mlp_grad(Ctx* c, const float* x, const int32_t* y, const float* w,
 Status launch_mlp_grad_tc(Ctx* c, const float* x, const int32_t* y, const float* w, int64_t n, float scale,
                           const float* theta, float* grad, uint32_t* err) {
   if (n == 0) return Status::ok();
-  const size_t smem = sizeof(TcGradSmem) + 1024;
+  const size_t smem = sizeof(TcGradSmem) + 128;
   SPLAT_CUDA(cudaFuncSetAttribute(mlp_grad_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int dev = 0, sms = 0;
   SPLAT_CUDA(cudaGetDevice(&dev));
   SPLAT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  // One CTA per SM: each holds all 512 tensor-memory columns.
-  const int64_t grid = std::min<int64_t>(ceil_div(n, kTcRows), (int64_t)sms);
+  // Two CTAs per SM: each holds half of the 512 tensor-memory columns.
+  const int64_t grid = std::min<int64_t>(ceil_div(n, kTcRows), (int64_t)(512 / kGradTmemCols) * sms);
   mlp_grad_tc_kernel<<<(unsigned)grid, kTcRows, smem, c->stream>>>(x, y, w, n, scale, theta, grad, err);
   c->launches.count++;
   SPLAT_LAUNCHED("mlp_grad_tc_kernel");
