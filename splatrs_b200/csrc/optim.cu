@@ -50,6 +50,9 @@ AdamArgs make_adam_args(uint64_t step, const splat_lr& lr) {
   a.eps = 1e-15f;
   a.c1 = 1.0f - powi_f(a.b1, (int)step);
   a.c2 = 1.0f - powi_f(a.b2, (int)step);
+  a.recip = a.c1 >= 0x1p-10f && a.c1 <= 1.0f && a.c2 >= 0x1p-10f && a.c2 <= 1.0f;
+  a.r1 = a.recip ? 1.0f / a.c1 : 0.0f;
+  a.r2 = a.recip ? 1.0f / a.c2 : 0.0f;
   // Plane 0: mean x y z, opacity; plane 1: quat; plane 2: log-scale x y z, pad;
   // plane 3: sh[0][0..3] (DC) and sh[1][0] (rest).
   const float L[4][4] = {{lr.mean, lr.mean, lr.mean, lr.opacity},

@@ -795,8 +795,9 @@ __device__ __forceinline__ void proj_grad_one(const GParams& g, const splat_came
 // the gradients are computed and while earlier planes are updated. Every thread copies and reads
 // its own Gaussian's values, so a thread waits for its own copies and for nobody else. Without
 // this each plane's three loads started after the previous plane's stores (187k Gaussians at SH
-// degree 3: 114 -> 97 us with one view, 100k in a batch of 8 views 184 -> 166 us). What is left is
-// arithmetic: the update's three divisions and square root per parameter.
+// degree 3: 114 -> 97 us with one view, 100k in a batch of 8 views 184 -> 166 us). With the update
+// in fused multiply-adds and looped over the planes (adam_planes below) 97 -> 77 and 166 -> 147 us,
+// where the streamed bytes alone take 41 and 22; issue slots are 62% busy.
 template <int NT, int kAhead>
 struct AdamStage {
   float4 p[kAhead][NT], m[kAhead][NT], v[kAhead][NT];
@@ -805,38 +806,62 @@ __device__ __forceinline__ void copy_async16(float4* smem, const float4* global)
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(global) : "memory");
 }
+// Plane q into slot s (= q % kAhead).
 template <int NT, int kAhead>
-__device__ __forceinline__ void adam_prefetch(AdamStage<NT, kAhead>& st, int q, const float4* p, const float4* m,
-                                              const float4* v, int64_t cap, int64_t i) {
+__device__ __forceinline__ void adam_prefetch(AdamStage<NT, kAhead>& st, int s, int q, const float4* p,
+                                              const float4* m, const float4* v, int64_t cap, int64_t i) {
   if (q < kPlanes) {
     const int64_t o = (int64_t)q * cap + i;
-    const int s = q % kAhead, t = threadIdx.x;
+    const int t = threadIdx.x;
     copy_async16(&st.p[s][t], p + o);
     copy_async16(&st.m[s][t], m + o);
     copy_async16(&st.v[s][t], v + o);
   }
   asm volatile("cp.async.commit_group;" ::: "memory");  // one group per plane, empty past the last
 }
-// Plane q's operands, once its group has landed (the kAhead - 1 younger ones may still fly).
+// Slot s's operands, once their group has landed (the kAhead - 1 younger ones may still fly).
 template <int NT, int kAhead>
-__device__ __forceinline__ void adam_take(const AdamStage<NT, kAhead>& st, int q, float4& p, float4& m, float4& v) {
+__device__ __forceinline__ void adam_take(const AdamStage<NT, kAhead>& st, int s, float4& p, float4& m, float4& v) {
   asm volatile("cp.async.wait_group %0;" ::"n"(kAhead - 1) : "memory");
-  const int s = q % kAhead, t = threadIdx.x;
+  const int t = threadIdx.x;
   p = st.p[s][t];
   m = st.m[s][t];
   v = st.v[s][t];
 }
+// Adam::step (adam.rs:77-161) on every plane of Gaussian i, gradient grad(q), in place; the
+// render copy follows the f32 master (round to nearest even). One plane per round of a loop
+// that isn't unrolled: unrolled 15 times, the update's 4 x 60 instructions a plane missed the
+// instruction cache.
+template <bool BF16, int NT, int kAhead, class Grad>
+__device__ __forceinline__ void adam_planes(AdamStage<NT, kAhead>& st, const AdamArgs& adam, float4* planes,
+                                            float4* adam_m, float4* adam_v, int64_t cap, int64_t i, uint2* bf,
+                                            const Grad& grad) {
+  int s = 0;
+#pragma unroll 1
+  for (int q = 0; q < kPlanes; q++) {
+    const int64_t o = (int64_t)q * cap + i;
+    float4 p, m, v;
+    adam_take(st, s, p, m, v);
+    adam_plane(adam, q, p, grad(q), m, v);
+    planes[o] = p;
+    adam_m[o] = m;
+    adam_v[o] = v;
+    adam_prefetch(st, s, q + kAhead, planes, adam_m, adam_v, cap, i);
+    if (BF16 && q > 0) bf[(int64_t)(q - 1) * cap + i] = pack_bf16x4(p);
+    s = s + 1 == kAhead ? 0 : s + 1;
+  }
+}
 
 // project_backward_one (project.rs:335-474), plus DensifyStats::accumulate
 // (densify.rs:36-60) when `stats` is given. With ADAM the 59 gradients never leave the
-// registers: Adam::step (adam.rs:77-161) updates the parameters in place and the moments m
+// SM: Adam::step (adam.rs:77-161) updates the parameters in place and the moments m
 // and v, over every plane (zero gradients still decay the moments, adam.rs:56-60).
 // Four blocks of 128 per SM: the 59 gradients and the streamed parameters and moments
 // would take 190-242 registers (8 warps per SM, too few to hide the memory latency of an
 // HBM-bound kernel); capped at 128 the kernel spills a few hundred bytes to L1 and runs
 // 22-23% faster (measured at 1M Gaussians: 0.606 -> 0.475 ms with Adam, 0.149 -> 0.115 ms
 // without).
-constexpr int kAdamAhead = 3;  // 3, 5, 7: 97, 98, 103 us for 187k Gaussians
+constexpr int kAdamAhead = 3;  // 5 and 7 were no faster; 3 leaves room for the gradient columns in 48 KB
 template <int DEG, bool ADAM, bool BF16>
 __global__ void __launch_bounds__(128, 4) project_bwd_kernel(const float4* __restrict__ planes, int64_t n, int64_t cap,
                                                           splat_camera cam_arg, splat_proj_opts opts,
@@ -856,10 +881,11 @@ __global__ void __launch_bounds__(128, 4) project_bwd_kernel(const float4* __res
   __shared__ AdamStage<128, ADAM ? kAdamAhead : 1> st;
   if (ADAM) {
 #pragma unroll
-    for (int q = 0; q < kAdamAhead; q++) adam_prefetch(st, q, planes, adam_m, adam_v, cap, i);
+    for (int q = 0; q < kAdamAhead; q++) adam_prefetch(st, q, q, planes, adam_m, adam_v, cap, i);
   }
   const splat_camera cam = sp ? sp->cam : cam_arg;
-  const AdamArgs adam = (ADAM && sp) ? sp->adam : adam_arg;
+  __shared__ AdamArgs adam;
+  if (ADAM && threadIdx.x == 0) adam = sp ? sp->adam : adam_arg;  // thread 0 is never past n
   const float4 g0 = pgrad[i], g1 = pgrad[cap + i], g2 = pgrad[2 * cap + i];
 
   if (stat_accum != nullptr) {
@@ -896,31 +922,26 @@ __global__ void __launch_bounds__(128, 4) project_bwd_kernel(const float4* __res
 #pragma unroll
     for (int q = 0; q < 12; q++) out[(3 + q) * cap + i] = make_float4(o_sh[4 * q], o_sh[4 * q + 1], o_sh[4 * q + 2], o_sh[4 * q + 3]);
   } else {
+    // The gradients wait in this thread's column (row 11, the pad, left out), so that the
+    // update can loop over the planes.
+    __shared__ float col[ADAM ? kPlanes * 4 - 1 : 1][128];
+    const int tid = threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < 3; k++) col[k][tid] = o_mean[k];
+    col[3][tid] = o_op;
+#pragma unroll
+    for (int k = 0; k < 4; k++) col[4 + k][tid] = o_q[k];
+#pragma unroll
+    for (int k = 0; k < 3; k++) col[8 + k][tid] = o_ls[k];
+#pragma unroll
+    for (int k = 0; k < 48; k++) col[11 + k][tid] = o_sh[k];
+    __syncthreads();  // `adam`
     // The parameters are read above only through `planes`; each element is read before
     // this thread writes it and no other thread touches Gaussian i.
-    float4* pw = const_cast<float4*>(planes);
-#pragma unroll
-    for (int q = 0; q < kPlanes; q++) {
-      float4 g;
-      if (q == 0)
-        g = make_float4(o_mean[0], o_mean[1], o_mean[2], o_op);
-      else if (q == 1)
-        g = make_float4(o_q[0], o_q[1], o_q[2], o_q[3]);
-      else if (q == 2)
-        g = make_float4(o_ls[0], o_ls[1], o_ls[2], 0.0f);
-      else
-        g = make_float4(o_sh[4 * (q - 3)], o_sh[4 * (q - 3) + 1], o_sh[4 * (q - 3) + 2], o_sh[4 * (q - 3) + 3]);
-      const int64_t o = (int64_t)q * cap + i;
-      float4 p, m, v;
-      adam_take(st, q, p, m, v);
-      adam_plane(adam, q, p, g, m, v);
-      pw[o] = p;
-      adam_m[o] = m;
-      adam_v[o] = v;
-      adam_prefetch(st, q + kAdamAhead, pw, adam_m, adam_v, cap, i);
-      // The render copy follows the f32 master (round to nearest even).
-      if (BF16 && q > 0) bf[(int64_t)(q - 1) * cap + i] = pack_bf16x4(p);
-    }
+    adam_planes<BF16>(st, adam, const_cast<float4*>(planes), adam_m, adam_v, cap, i, bf, [&](int q) {
+      const int r = 4 * q - (q > 2);
+      return make_float4(col[r][tid], col[r + 1][tid], col[r + 2][tid], q == 2 ? 0.0f : col[r + 3][tid]);
+    });
   }
 }
 
@@ -1114,7 +1135,9 @@ __global__ void __launch_bounds__(kBatchBwdThreads) project_bwd_batch_adam_kerne
   const int tid = threadIdx.x;
   __shared__ AdamStage<kBatchBwdThreads, kBatchAhead> st;
 #pragma unroll
-  for (int q = 0; q < kBatchAhead; q++) adam_prefetch(st, q, planes, adam_m, adam_v, cap, i);
+  for (int q = 0; q < kBatchAhead; q++) adam_prefetch(st, q, q, planes, adam_m, adam_v, cap, i);
+  __shared__ AdamArgs adam;
+  if (tid == 0) adam = bt->adam;  // never past n
 #pragma unroll
   for (int f = 0; f < kPlanes * 4; f++) acc[f][tid] = 0.0f;
   GParams g;
@@ -1153,20 +1176,10 @@ __global__ void __launch_bounds__(kBatchBwdThreads) project_bwd_batch_adam_kerne
 #pragma unroll
     for (int q = 0; q < 48; q++) acc[12 + q][tid] += pgr.sh[q];
   }
-  const AdamArgs adam = bt->adam;
-#pragma unroll
-  for (int q = 0; q < kPlanes; q++) {
-    const float4 gq = make_float4(acc[4 * q][tid], acc[4 * q + 1][tid], acc[4 * q + 2][tid], acc[4 * q + 3][tid]);
-    const int64_t o = (int64_t)q * cap + i;
-    float4 p, m, v;
-    adam_take(st, q, p, m, v);
-    adam_plane(adam, q, p, gq, m, v);
-    planes[o] = p;
-    adam_m[o] = m;
-    adam_v[o] = v;
-    adam_prefetch(st, q + kBatchAhead, planes, adam_m, adam_v, cap, i);
-    if (BF16 && q > 0) bf[(int64_t)(q - 1) * cap + i] = pack_bf16x4(p);
-  }
+  __syncthreads();  // `adam`
+  adam_planes<BF16>(st, adam, planes, adam_m, adam_v, cap, i, bf, [&](int q) {
+    return make_float4(acc[4 * q][tid], acc[4 * q + 1][tid], acc[4 * q + 2][tid], acc[4 * q + 3][tid]);
+  });
 }
 
 Status launch_project_bwd_batch_adam(Ctx* c, float* planes, float* m, float* v, int64_t n, int64_t cap,
