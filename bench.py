@@ -190,8 +190,6 @@ def unit_peaks(ctx, local):
 # Algorithmic work per unit (fixed constants): bytes for the HBM-bound stages.
 PROJ_FWD_BYTES = 236 + 64          # parameters read + projection record written, per Gaussian
 PROJ_BWD_BYTES = 236 + 36 + 236    # parameters + screen gradients read, parameter gradients written
-SORT_BYTES_PER_KEY_PASS = 24       # one read and one write of a (u64 key, u32 value) pair
-EMIT_BYTES_PER_ENTRY = 12          # key + value written
 RASTER_FWD_BYTES_PER_PIXEL = 20    # image (12) + final T (4) + n_contrib (4) written
 RASTER_BWD_BYTES_PER_PIXEL = 20    # dL/dpix (12) + final T (4) + n_contrib (4) read
 RASTER_BYTES_PER_ENTRY = 52        # sorted index (4) + record gather (48)
@@ -208,7 +206,7 @@ RASTER_FWD_FLOP_PER_PAIR = 20
 RASTER_BWD_FLOP_PER_PAIR = 50
 RASTER_FWD_SFU_PER_PAIR = 1        # one exp
 RASTER_BWD_SFU_PER_PAIR = 2        # one exp, one reciprocal (the transmittance division)
-BIN_BYTES_PER_ENTRY = 40 + 24      # key emission (key 8 + value 4 + entry Gaussian 4, Proj read) + sort (24)
+BIN_BYTES_PER_ENTRY = 36 + 16      # key emission (packed key 8 + entry Gaussian 4, Proj read 24) + sort (16)
 
 
 def stage_rooflines(stage_ms, n, entries, pairs_fwd, pairs_bwd, pixels, hbm_gbs, fp32_tflops, mufu_gops):

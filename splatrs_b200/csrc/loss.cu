@@ -395,7 +395,7 @@ __global__ void __launch_bounds__(kLossThreads) ssim_bwd_kernel(const float* __r
 // Small views: a block takes one channel of a 32 x 16 tile, and each blur pass gives a thread
 // kRun consecutive outputs of a row (then of a column) and streams their kRun + 10 inputs once.
 // Such a view has too few 32 x 32 tiles of three channels for the SMs, so its time is one
-// block's chain: 256x256 42 -> 18.6 us, 64x48 37 -> 13.5 us (runs of 8 outputs 22.6 and 18.5).
+// block's chain: 256x256 42 -> 18.5 us, 64x48 37 -> 12.6 us (runs of 8 outputs 22.6 and 18.5).
 // ---------------------------------------------------------------------------------------
 constexpr int kRun = 4;
 constexpr int kTileW = kLossTile;
