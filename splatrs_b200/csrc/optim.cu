@@ -14,9 +14,13 @@
 
 namespace splat {
 
+// Streams 1680 bytes a Gaussian: 1M take 257 us (6.5 TB/s), whatever the share of zero moments;
+// with the operators in adam_update 305 us, and 388 where half of the moments are zero. The
+// arguments stay in the parameter space, which a plane can index (a copy per thread in local
+// memory cost 86 us).
 __global__ void __launch_bounds__(256) adam_kernel(float4* __restrict__ p, const float4* __restrict__ g,
                                                    float4* __restrict__ m, float4* __restrict__ v, int64_t n,
-                                                   int64_t cap, AdamArgs a) {
+                                                   int64_t cap, const __grid_constant__ AdamArgs a) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t total = (int64_t)kPlanes * n;
   if (t >= total) return;
