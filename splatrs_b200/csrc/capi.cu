@@ -167,7 +167,6 @@ SPLAT_API int splat_ctx_destroy(splat_ctx* ctx) {
   cudaSetDevice(ctx->c.device);
   cudaStreamSynchronize(ctx->c.stream);
   arena_free(&ctx->c);
-  download_free(&ctx->c);
   if (ctx->c.host_small) cudaFreeHost(ctx->c.host_small);
   cudaSetDevice(prev);
   delete ctx;

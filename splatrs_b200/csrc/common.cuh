@@ -90,7 +90,6 @@ struct RasterConfig {
 // Most tiles any supported shape gives an image (8x8): sizes per-tile buffers for all.
 inline uint32_t max_tiles(uint32_t width, uint32_t height) { return ((width + 7) / 8) * ((height + 7) / 8); }
 
-struct Download;
 struct Ctx {
   int device = 0;
   RasterConfig raster;
@@ -99,7 +98,6 @@ struct Ctx {
   LaunchCounter launches;
   std::string last_error;
   int sm_count = 148;
-  Download* download = nullptr;  // slots of download_records, made on its first use
   // Mapped pinned host memory for small read-backs: kernels store into it through
   // host_small_dev, so a read-back never queues on a copy engine behind large transfers.
   void* host_small = nullptr;

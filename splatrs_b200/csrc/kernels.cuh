@@ -46,7 +46,6 @@ Status launch_params_from_aos(Ctx* c, const float* aos, int64_t n, float* planes
 Status launch_params_to_aos(Ctx* c, const float* planes, int64_t n, int64_t cap, float* aos);
 // Records of all n Gaussians into a host array (download.cu); synchronises.
 Status download_records(Ctx* c, const float* planes, int64_t n, int64_t cap, float* aos_host);
-void download_free(Ctx* c);
 
 Status launch_project_fwd(Ctx* c, const float* planes, int64_t n, int64_t cap, const splat_camera& cam,
                           const splat_proj_opts& opts, float* proj, uint32_t* num_tiles, uint32_t* depth_range,
