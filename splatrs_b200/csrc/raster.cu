@@ -896,17 +896,20 @@ constexpr float kSigmaEdge = 1e-4f;
 //    accumulator by 0 + 1, and its contributions are exactly zero. What a pixel contributes
 //    to the entry's gradients is two numbers: h = gauss dL/dalpha and w = alpha T.
 // 3. Lane (e, q) sums h {1, dx, dx^2} (dy and its products are constant over a row), w {1,
-//    dL/dr, dL/dg, dL/db} and the two absolute gradients over its row; the 12 slots follow by
-//    linear combination (with -dsigma = opacity h), two exchange stages add the entry's four
-//    lanes, and one float4 vector atomic per gradient plane adds them to global memory.
+//    dL/dr, dL/dg, dL/db}, h (A dx + B dy, B dx + C dy) and its absolute values over its row; the
+//    12 slots follow by linear combination (with -dsigma = opacity h), two exchange stages add
+//    the entry's four lanes, and one float4 vector atomic per gradient plane adds them to global
+//    memory. The mean's gradient is summed pixel by pixel, not as A sum(h dx) + B sum(h dy): for
+//    an elongated, tilted Gaussian these two nearly cancel, which amplified the sums' rounding
+//    (axes 50 and 0.1 pixels: 1.5 times the error of summing in the reference's order, now 0.7).
 //
 // The phases hand (gauss) and (h, w) over in two 8 x 32 arrays of pairs in shared memory.
 // Against one pixel pair per lane for everything (records broadcast from shared memory with
 // each scalar duplicated, a 13-shuffle reduction of 12 slots over the warp for every entry)
 // this takes about 130 instead of 185 warp instructions per entry. Bound by latency and issue
 // (63% of the issue slots, FMA pipe 48%, shared-memory reads 60%; DRAM 3% of its peak).
-// Time: 1M Gaussians at 1920x1080 975 -> 653 us, 187k clustered at 1297x840 377 -> 256, 34k at
-// 256x256 164 -> 78, 20k wide ones at 1386x1080 163 -> 115. kCount adds the evaluated-pair
+// Time: 1M Gaussians at 1920x1080 975 -> 661 us, 187k clustered at 1297x840 377 -> 262, 34k at
+// 256x256 164 -> 79, 20k wide ones at 1386x1080 163 -> 117. kCount adds the evaluated-pair
 // counter (untimed diagnostics only).
 constexpr int kGroup = 8;      // entries per round of the three phases
 constexpr int kBwdStage = 16;  // entries staged per copy
@@ -1216,7 +1219,7 @@ __global__ void __launch_bounds__(32 * BwdShape<TW, TH>::kWarps, kSmWarps / BwdS
         __syncwarp();
         // ---- Phase 3
         const f2 bdy = f2_mul(f2_splat(B), dy);
-        f2 h0 = f2_splat(0.0f), h1 = h0, h2 = h0, w0 = h0, wr = h0, wg = h0, wb = h0;
+        f2 h0 = f2_splat(0.0f), h1 = h0, h2 = h0, gx = h0, gy = h0, w0 = h0, wr = h0, wg = h0, wb = h0;
         float ax = 0.0f, ay = 0.0f;
         f2 dx = f2_splat(px0 - r0.x);
 #pragma unroll
@@ -1233,11 +1236,14 @@ __global__ void __launch_bounds__(32 * BwdShape<TW, TH>::kWarps, kSmWarps / BwdS
           wr = f2_fma(w, f2_make(d01.x, d01.y), wr);
           wg = f2_fma(w, f2_make(d01.z, d01.w), wg);
           wb = f2_fma(w, f2_make(d2.x, d2.y), wb);
+          const f2 hmx = f2_mul(h, f2_fma(f2_splat(A), dx, bdy)), hmy = f2_mul(h, f2_fma(f2_splat(B), dx, cdy));
+          gx = f2_add(gx, hmx);
+          gy = f2_add(gy, hmy);
           float lo, hi;
-          f2_split(f2_mul(h, f2_fma(f2_splat(A), dx, bdy)), lo, hi);
+          f2_split(hmx, lo, hi);
           ax += fabsf(lo);
           ax += fabsf(hi);
-          f2_split(f2_mul(h, f2_fma(f2_splat(B), dx, cdy)), lo, hi);
+          f2_split(hmy, lo, hi);
           ay += fabsf(lo);
           ay += fabsf(hi);
           dx = f2_add(dx, f2_splat(1.0f));
@@ -1247,14 +1253,16 @@ __global__ void __launch_bounds__(32 * BwdShape<TW, TH>::kWarps, kSmWarps / BwdS
         float v[kSlots], lo, hi, dy0, dy1;
         f2_split(dy, dy0, dy1);
         f2_split(h0, lo, hi);
-        const float sy = __fmaf_rn(dy1, hi, dy0 * lo), syy = __fmaf_rn(dy1 * dy1, hi, (dy0 * dy0) * lo);
+        const float syy = __fmaf_rn(dy1 * dy1, hi, (dy0 * dy0) * lo);
         v[5] = lo + hi;
         f2_split(h1, lo, hi);
-        const float sx = lo + hi, sxy = __fmaf_rn(dy1, hi, dy0 * lo);
+        const float sxy = __fmaf_rn(dy1, hi, dy0 * lo);
         f2_split(h2, lo, hi);
         const float sxx = lo + hi;
-        v[0] = opacity * __fmaf_rn(A, sx, B * sy);
-        v[1] = opacity * __fmaf_rn(B, sx, r1.x * sy);
+        f2_split(gx, lo, hi);
+        v[0] = opacity * (lo + hi);
+        f2_split(gy, lo, hi);
+        v[1] = opacity * (lo + hi);
         v[2] = -0.5f * opacity * sxx;
         v[3] = -opacity * sxy;
         v[4] = -0.5f * opacity * syy;
