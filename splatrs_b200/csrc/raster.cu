@@ -371,19 +371,21 @@ __device__ __forceinline__ void copy_async16(float4* smem, const float4* global)
 }
 __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// One warp's pass over a scanned list: the entries whose mask has the warp's bit, in order,
-// queued (as list indices) and staged STAGE (at most 32) at a time.
+// One warp's pass over a scanned list: the entries from `first` on whose mask has the warp's bit,
+// in order, queued (as list indices) and staged STAGE (at most 32) at a time.
 template <typename Mask, int STAGE>
 struct Stager {
   const TileList<Mask>* list;
   uint32_t cnt, pos, head, tail, bit;
   uint16_t* queue;
-  __device__ __forceinline__ void start(const TileList<Mask>* l, uint32_t cnt_, uint32_t bit_, uint16_t* q) {
+  __device__ __forceinline__ void start(const TileList<Mask>* l, uint32_t first, uint32_t cnt_, uint32_t bit_,
+                                        uint16_t* q) {
     list = l;
     cnt = cnt_;
     bit = bit_;
     queue = q;
-    pos = head = tail = 0;
+    pos = first;
+    head = tail = 0;
   }
   // Starts the copies of the next stage's records, part p of entry i to s + p * stride + i
   // (four lanes per record: one 64-byte line each); returns how many entries, and through *g
@@ -524,7 +526,7 @@ __global__ void __launch_bounds__(32 * FwdShape<TW, TH>::kWarps, 32 / FwdShape<T
     wk.template barrier<Shape::kTiles>();
     if (__all_sync(0xffffffffu, done)) continue;
     Stager<typename W::Mask, kStage> stager;
-    stager.start(&list, cnt, wk.sub, st.queue);
+    stager.start(&list, 0, cnt, wk.sub, st.queue);
     uint32_t buf = 0, g = 0, index = 0;
     uint32_t m = stager.fetch(rec, st.s[0][0], kStage + 1, &g, &index);
     while (m) {
@@ -908,7 +910,7 @@ constexpr float kSigmaEdge = 1e-4f;
 // each scalar duplicated, a 13-shuffle reduction of 12 slots over the warp for every entry)
 // this takes about 130 instead of 185 warp instructions per entry. Bound by latency and issue
 // (63% of the issue slots, FMA pipe 48%, shared-memory reads 60%; DRAM 3% of its peak).
-// Time: 1M Gaussians at 1920x1080 975 -> 661 us, 187k clustered at 1297x840 377 -> 262, 34k at
+// Time: 1M Gaussians at 1920x1080 975 -> 666 us, 187k clustered at 1297x840 377 -> 257, 34k at
 // 256x256 164 -> 79, 20k wide ones at 1386x1080 163 -> 117. kCount adds the evaluated-pair
 // counter (untimed diagnostics only).
 constexpr int kGroup = 8;      // entries per round of the three phases
@@ -1096,7 +1098,9 @@ __global__ void __launch_bounds__(32 * BwdShape<TW, TH>::kWarps, kSmWarps / BwdS
   const float px0 = (float)wk.bx + 0.5f;
   const f2 pyq = f2_make((float)(wk.by + q) + 0.5f, (float)(wk.by + q + 4u) + 0.5f);
 
-  // Entries at or past every pixel's n_contrib contribute nothing to the tile.
+  // Entries at or past every pixel's n_contrib contribute nothing: the tile's list is scanned from
+  // its last contributor on, and the warp takes up the walk at its own (one that saturates early
+  // beside one that doesn't has most of the list behind it).
   const uint32_t warp_last = __reduce_max_sync(0xffffffffu, max(last[0], last[1]));
   uint32_t min_last;  // over the image's pixels (the others are in no rectangle)
   {
@@ -1114,7 +1118,8 @@ __global__ void __launch_bounds__(32 * BwdShape<TW, TH>::kWarps, kSmWarps / BwdS
     wk.scan(list, n - 1u - first, -1, total);
     wk.template barrier<Shape::kTiles>();
     Stager<typename W::Mask, kBwdStage> stager;
-    stager.start(&list, total, wk.sub, st.queue);
+    const uint32_t past = n - min(n, first + warp_last);  // of this scan's entries, those past the warp's last
+    stager.start(&list, past, total, wk.sub, st.queue);
     uint32_t buf = 0, next_g = 0, next_index = 0;
     uint32_t m = stager.fetch(rec, st.s[0][0], kBwdStage, &next_g, &next_index);
     while (m) {

@@ -89,3 +89,33 @@ def test_lists_at_the_edges_of_a_walk(ctx, cr_math, tile, n, opacity, special):
         for got, want in ((gg, og), (ga, oa)):
             scale = np.maximum(np.abs(want).max(0), 1e-30)
             assert (np.abs(got - want).max(0) / scale).max() < 1e-3
+
+
+@pytest.mark.parametrize("tile", [(16, 16), (8, 8), (16, 32)])
+@pytest.mark.parametrize("n", [40, 1100, 2300])
+def test_warps_that_saturate_early(ctx, cr_math, tile, n):
+    """Opaque entries in front close the pixels around one corner of a tile, while those of the
+    other corners go through the whole list, over one, two and three scans of it: the backward's
+    warps start at places of their own."""
+    p = projections(n, 0.4 / np.sqrt(n), 500 + n)
+    p[:12, :5] = (4.0, 4.0, 0.02, 0.0, 0.02)
+    p[:12, 5], p[:12, 6], p[:12, 7] = 0.5 + 0.01 * np.arange(12), 3.0, 0.99
+    dimage = np.random.default_rng(n).normal(0, 1, SIZE[0] * SIZE[1] * 3).astype(np.float32)
+    ob = O.bin(p, *SIZE)
+    img, ft, nc, _ = O.rasterize_forward(p, ob, *SIZE, BG)
+    og, oa, opairs = O.rasterize_backward(p, ob, *SIZE, BG, ft, nc, dimage)
+    assert nc.min() <= 8 and nc.max() > 0.9 * n
+    ctx.raster_config = (*tile, 256, 2)
+    try:
+        proj = G.proj_from_reference(ctx, dev(p), *SIZE)
+        b = G.bin(ctx, proj)
+        out = G.rasterize_forward(ctx, proj, b, BG)
+        got_pairs = torch.zeros(1, dtype=torch.int64, device="cuda")
+        pgrad = G.rasterize_backward(ctx, proj, b, BG, out, dev(dimage), pairs=got_pairs)
+    finally:
+        ctx.raster_config = (16, 16, 256, 2)
+    assert (bits(out.image.cpu().numpy()) == bits(img)).all()
+    assert int(got_pairs.item()) == opairs
+    for got, want in zip((v.cpu().numpy() for v in G.pgrad_to_reference(pgrad, n)), (og, oa)):
+        scale = np.maximum(np.abs(want).max(0), 1e-30)
+        assert (np.abs(got - want).max(0) / scale).max() < 1e-3
