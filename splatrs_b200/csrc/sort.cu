@@ -907,7 +907,7 @@ __global__ void __launch_bounds__(kRangeThreads) tile_ranges_dev_kernel(DevBuffe
 
 size_t dev_sort_scratch_bytes(int64_t E_cap) {
   const int64_t cap = std::max<int64_t>(E_cap, 1);
-  return (size_t)cap * 24 + sort_ctl_bytes(cap) + 6 * 256;  // 5 pieces, 256-aligned
+  return (size_t)cap * 24 + sort_ctl_bytes(cap) + 6 * 256;  // 5 pieces, 256-aligned wherever the scratch starts
 }
 
 template <bool kPacked, typename W>
@@ -917,7 +917,9 @@ static Status sort_entries_dev(Ctx* c, const float* proj, const uint32_t* entry_
                                uint32_t* ranges, uint32_t* overflow, const BatchTable* bt, int64_t n_view) {
   const int64_t cap = std::max<int64_t>(E_cap, 1);
   const uint64_t tiles = sort_tiles(cap);
-  // Carve the scratch (256-byte aligned pieces).
+  // Carve the scratch (256-byte aligned pieces: the caller's base may have any alignment, and the
+  // range kernel reads 16 bytes at a time).
+  scratch = reinterpret_cast<void*>((reinterpret_cast<uintptr_t>(scratch) + 255) & ~(uintptr_t)255);
   auto carve = [&](size_t bytes) {
     void* p = scratch;
     scratch = static_cast<char*>(scratch) + ((bytes + 255) & ~(size_t)255);
