@@ -272,9 +272,10 @@ SPLAT_API int splat_bin_sort(splat_ctx* ctx, const float* proj_dev, const uint32
  * memory (*num_entries_dev, uint64) instead of returning it, and splat_bin_sort_device
  * reads it there. Buffers are sized for `capacity` entries: gauss_dev holds capacity
  * values and scratch_dev splat_bin_sort_device_scratch_bytes(capacity) bytes, at any
- * alignment. When the count exceeds capacity the call sorts only the first `capacity` entries
- * and sets *overflow_dev to 1 (it is never cleared here): the view must then be redone with
- * larger buffers. Otherwise gauss_dev and tile_range_dev equal splat_bin_sort's. */
+ * alignment (never fewer for a larger capacity, so scratch for one serves all smaller ones).
+ * When the count exceeds capacity the call sorts only the first `capacity` entries and sets
+ * *overflow_dev to 1 (it is never cleared here): the view must then be redone with larger
+ * buffers. Otherwise gauss_dev and tile_range_dev equal splat_bin_sort's. */
 SPLAT_API int splat_bin_count_device(splat_ctx* ctx, const uint32_t* num_tiles_dev, int64_t n,
                                      uint32_t* entry_offset_dev, uint64_t* num_entries_dev);
 SPLAT_API size_t splat_bin_sort_device_scratch_bytes(int64_t capacity);

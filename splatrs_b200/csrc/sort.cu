@@ -905,9 +905,14 @@ __global__ void __launch_bounds__(kRangeThreads) tile_ranges_dev_kernel(DevBuffe
   tile_ranges_body(reinterpret_cast<const uint32_t*>((lay.passes - 1) & 1 ? b.ka : b.kb), lay.E, ranges);
 }
 
+// Never less for a larger capacity, so that scratch for one serves every smaller one: the look-back
+// words shrink where larger tiles come in (65,536 keys take 64 tiles of 1,024, 65,537 take 33 of
+// 2,048), so a size covers the largest sort of each smaller shape too.
 size_t dev_sort_scratch_bytes(int64_t E_cap) {
   const int64_t cap = std::max<int64_t>(E_cap, 1);
-  return (size_t)cap * 24 + sort_ctl_bytes(cap) + 6 * 256;  // 5 pieces, 256-aligned wherever the scratch starts
+  size_t ctl = sort_ctl_bytes(cap);
+  for (const int64_t last : {kSmallSortKeys, kMidSortKeys}) ctl = std::max(ctl, sort_ctl_bytes(std::min(cap, last)));
+  return (size_t)cap * 24 + ctl + 6 * 256;  // 5 pieces, 256-aligned wherever the scratch starts
 }
 
 template <bool kPacked, typename W>

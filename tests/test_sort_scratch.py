@@ -1,5 +1,6 @@
-"""The caller's scratch of the device-driven sort (splat_bin_sort_device): any alignment, and
-nothing written outside of the bytes that splat_bin_sort_device_scratch_bytes asks for."""
+"""The caller's scratch of the device-driven sort (splat_bin_sort_device): any alignment, scratch
+for one capacity serves every smaller one, and nothing is written outside of the bytes that
+splat_bin_sort_device_scratch_bytes asks for."""
 import numpy as np
 import pytest
 import torch
@@ -43,5 +44,21 @@ def sort_in(ctx, n, capacity, offset, size):
 def test_scratch_at_any_alignment(n, capacity, offset):
     ctx = G.Context(0)
     got, want, whole = sort_in(ctx, n, capacity, offset, need(capacity))
+    assert torch.equal(got, want) and whole
+    ctx.close()
+
+
+def test_scratch_never_shrinks_with_the_capacity():
+    edges = [c + d for c in (0, 1, 1024, 2048, 4096, 1 << 16, 1 << 17, 3 << 18, 3 << 19, 1 << 30) for d in (-1, 0, 1)]
+    sizes = sorted({c for c in edges if c >= 0} | set(range(1, 2_000_000, 997)) | {800_000, 830_000})
+    asked = [need(c) for c in sizes]
+    assert all(a <= b for a, b in zip(asked, asked[1:]))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("capacity,larger", [(65536, 65537), (65536, 70000), (786432, 786433), (786432, 800000)])
+def test_scratch_of_a_larger_capacity(capacity, larger):
+    ctx = G.Context(0)
+    got, want, whole = sort_in(ctx, capacity, capacity, 0, need(larger))
     assert torch.equal(got, want) and whole
     ctx.close()
