@@ -178,7 +178,9 @@ inline Status launch_chained(Ctx* c, const char* what, void (*kernel)(P...), dim
     cfg.numAttrs = 1;
   }
   c->launches.count++;
-  return cuda_status(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...), what);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  if (e != cudaSuccess) cudaGetLastError();  // reported here, not by the next launch's check as well
+  return cuda_status(e, what);
 }
 #endif
 
