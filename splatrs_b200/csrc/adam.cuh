@@ -52,7 +52,8 @@ static __device__ __noinline__ float adam_quotient(float m, float v, float lr, f
 // small operands send the division and the square root down their long way, lane by lane; the
 // steps above need none of it in
 //   v = 0 or 2^-126 <= v <= 2^60 (scaled by 2^80 where small, so that remainders are exact),
-//   m = 0 or 2^-90 <= |m| <= 2^60 with |lr m_hat| >= 2^-90,
+//   m = 0 or 2^-90 <= |m| <= 2^60 with 2^-90 <= |lr m_hat| <= 2^60 (so that no quotient and no
+//   remainder overflows: |lr m_hat| / 1e-15 stays below 2^110),
 // and where m is smaller, but the quotient below 2^-27 |p|, p stays what it is for any
 // quotient of that size. False for everything else: q is then to come from adam_quotient.
 __device__ __forceinline__ bool adam_moments(float p, float g, float& m, float& v, float lr, const AdamArgs& a,
@@ -67,7 +68,7 @@ __device__ __forceinline__ bool adam_moments(float p, float g, float& m, float& 
   q = m == 0.0f ? num : q;
   const float am = fabsf(m), ap = fabsf(p);
   const bool v_ok = v == 0.0f || (v >= 0x1p-126f && v <= 0x1p60f);
-  const bool m_ok = m == 0.0f || (fminf(am, fabsf(num)) >= 0x1p-90f && am <= 0x1p60f) ||
+  const bool m_ok = m == 0.0f || (fminf(am, fabsf(num)) >= 0x1p-90f && fmaxf(am, fabsf(num)) <= 0x1p60f) ||
                     (ap >= 0x1p-60f && fabsf(q) < 0x1p-27f * ap);
   return v_ok & m_ok & ((__float_as_uint(den) & 0x7FFFFFu) != 0x7FFFFFu);
 }

@@ -46,3 +46,22 @@ def test_adam_range_bit_exact(ctx, step, lo, hi):
         nan = np.isnan(want)
         assert np.array_equal(np.isnan(got), nan)
         assert np.array_equal(got.view(np.uint32)[~nan], want.view(np.uint32)[~nan])
+
+
+@pytest.mark.parametrize("rate", [1e-30, 1.0, 1e6, 1e25, 3e38])
+def test_adam_rate_bit_exact(ctx, rate):
+    """Rates and moments whose step overflows to an infinity, or is lost, are the oracle's too."""
+    n = 2000
+    rng = np.random.default_rng(17)
+    p, g = _spread(rng, (n, 59), -20, 5, 0.1), np.zeros((n, 59), np.float32)
+    m, v = _spread(rng, (n, 59), -60, 60, 0.1), np.abs(_spread(rng, (n, 59), -60, 60, 0.5))
+    lr = LearningRates(*[rate] * 6)
+    t = [G.params_to_planes(ctx, torch.from_numpy(a).cuda(), None) for a in (p, g, m, v)]
+    G.adam_step(ctx, *t, n, n, 3, lr)
+    with np.errstate(all="ignore"):
+        O.adam_step(p, g, m, v, 2, np.full(6, rate, np.float32))
+    for got, want in ((t[0], p), (t[2], m), (t[3], v)):
+        got = G.planes_to_params(ctx, got, n, n).cpu().numpy()
+        nan = np.isnan(want)
+        assert np.array_equal(np.isnan(got), nan)
+        assert np.array_equal(got.view(np.uint32)[~nan], want.view(np.uint32)[~nan])
