@@ -757,6 +757,19 @@ static Status launch_pass(Ctx* c, void (*kernel)(P...), size_t smem, uint64_t ti
   return launch_chained(c, "radix_onesweep_kernel", kernel, (uint32_t)tiles, S::kThreads, smem, args...);
 }
 
+// SPLAT_PASS with the tile shape of a sort of `keys` (sort_tiles); 64-bit look-back words only
+// come with more keys than the smaller shapes take.
+#define SPLAT_PASS_BY_SIZE(keys)       \
+  if constexpr (sizeof(W) == 8) {      \
+    SPLAT_PASS(SortLarge);             \
+  } else if (keys <= kSmallSortKeys) { \
+    SPLAT_PASS(SortSmall);             \
+  } else if (keys <= kMidSortKeys) {   \
+    SPLAT_PASS(SortMid);               \
+  } else {                             \
+    SPLAT_PASS(SortLarge);             \
+  }
+
 template <bool kPacked, typename W>
 static Status sort_entries(Ctx* c, const float* proj, const uint32_t* entry_offset, int64_t n, const KeyLayout& lay,
                            const uint32_t* depth_range, uint32_t depth_min, uint32_t tiles_x, const SortBuffers& buf,
@@ -782,12 +795,7 @@ static Status sort_entries(Ctx* c, const float* proj, const uint32_t* entry_offs
 #define SPLAT_PASS(S)                                                                                          \
   SPLAT_TRY((launch_pass<S>(c, radix_onesweep_kernel<S, kPacked, W>, onesweep_smem<S, kPacked>(), sort_tiles(E), \
                             ka, va, E, p, ctl, err, out)))
-    if (sizeof(W) == 4 && E <= kSmallSortKeys)
-      SPLAT_PASS(SortSmall);
-    else if (sizeof(W) == 4 && E <= kMidSortKeys)
-      SPLAT_PASS(SortMid);
-    else
-      SPLAT_PASS(SortLarge);
+    SPLAT_PASS_BY_SIZE(E)
 #undef SPLAT_PASS
     std::swap(ka, kb);
     std::swap(va, vb);
@@ -949,12 +957,7 @@ static Status sort_entries_dev(Ctx* c, const float* proj, const uint32_t* entry_
 #define SPLAT_PASS(S)                                                                                          \
   SPLAT_TRY((launch_pass<S>(c, radix_onesweep_dev_kernel<S, kPacked, W>, onesweep_smem<S, kPacked>(), tiles, b, \
                             E_dev, E_cap, dr, tbits, vbits, pass, ctl, tiles, overflow, gauss_out)))
-    if (sizeof(W) == 4 && cap <= kSmallSortKeys)
-      SPLAT_PASS(SortSmall);
-    else if (sizeof(W) == 4 && cap <= kMidSortKeys)
-      SPLAT_PASS(SortMid);
-    else
-      SPLAT_PASS(SortLarge);
+    SPLAT_PASS_BY_SIZE(cap)
 #undef SPLAT_PASS
   }
   SPLAT_TRY(launch_chained(c, "tile_ranges_dev_kernel", tile_ranges_dev_kernel, ceil_div(cap, 4 * kRangeThreads),
@@ -979,5 +982,7 @@ Status launch_bin_sort_dev(Ctx* c, const float* proj, const uint32_t* entry_offs
   return packed ? SPLAT_SORT(true, uint32_t) : SPLAT_SORT(false, uint32_t);
 #undef SPLAT_SORT
 }
+
+#undef SPLAT_PASS_BY_SIZE
 
 }  // namespace splat
