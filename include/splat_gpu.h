@@ -407,8 +407,8 @@ SPLAT_API int splat_mlp_adam(splat_ctx* ctx, float* theta_dev, const float* grad
  * images, final transmittances and, up to summation order, gradients (each entry's pixel
  * rectangle is first narrowed to its 16-pixel tile rectangle). Chunk depth: entries
  * that the one-pixel-per-thread backward stages in shared memory per round, 32, 64, 128 or
- * 256 (the forward's and the two-pixel backward's warps walk their lists by themselves). Pixels per thread of the
- * backward: 1 or 2 (a warp then covers 8x8 pixels). Default 16x16, 256, 2.
+ * 256 (no other kernel depends on it). Pixels per thread of the backward: 1 or 2 (a warp
+ * then covers 8x8 pixels). Default 16x16, 256, 2.
  *   splat_raster_candidates: writes the supported (tile_w, tile_h, chunk,
  *     pixels_per_thread) quadruples to out (4 values each; out may be NULL) and returns
  *     how many (24).
@@ -417,7 +417,8 @@ SPLAT_API int splat_mlp_adam(splat_ctx* ctx, float* theta_dev, const float* grad
  *     one view (dimage_dev: dL/dimage, H*W*3) under every candidate, `reps` timed passes
  *     each after an untimed one, sets the fastest on the context and writes the mean
  *     milliseconds per pass of every candidate to ms_out (one per candidate) and the pick
- *     to picked (4).
+ *     to picked (4). With two pixels per thread the chunk depth changes no kernel: each
+ *     tile shape is timed once, at 256, and its time stands for the other depths.
  *     Synchronises; changes no caller buffer.
  * -------------------------------------------------------------------------------------- */
 SPLAT_API int32_t splat_raster_candidates(uint32_t* out);

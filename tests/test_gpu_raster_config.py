@@ -164,6 +164,10 @@ def test_autotune_render_times_every_candidate(ctx, config):
         assert all(np.isfinite(v) and v > 0 for v in res["ms"].values())
         assert res["picked"] in CANDS and ctx.raster_config == res["picked"]
         assert res["ms"][res["picked"]] == min(res["ms"].values())
+        # The chunk depth changes no kernel of two pixels per thread: one time, the deepest picked.
+        for w, h in ((8, 8), (16, 16), (16, 32)):
+            assert len({res["ms"][(w, h, ch, 2)] for ch in (32, 64, 128, 256)}) == 1
+        assert res["picked"][3] == 1 or res["picked"][2] == 256
         proj = G.project_all(ctx, planes, n, n, cam, opts)
         b = G.bin(ctx, proj)
         got = G.rasterize_forward(ctx, proj, b, [0.0, 0.0, 0.0]).image.cpu().numpy()
