@@ -39,6 +39,16 @@ CRM_HD double bits_to_double(uint64_t b) {
 #endif
 }
 
+CRM_HD uint32_t float_to_bits(float f) {
+#if defined(__CUDA_ARCH__)
+  return __float_as_uint(f);
+#else
+  uint32_t b;
+  __builtin_memcpy(&b, &f, 4);
+  return b;
+#endif
+}
+
 CRM_HD uint64_t double_to_bits(double d) {
 #if defined(__CUDA_ARCH__)
   return (uint64_t)__double_as_longlong(d);
@@ -114,9 +124,8 @@ CRM_HD float exp_grid_finish(float t, double e) {
 
 CRM_HD float expf_cr_grid(float s, const double* tab) {
   const float m = fmaf(s, 128.0f, kExpGridMagic);
-  const float nf = m - kExpGridMagic;
-  const float t = fmaf(nf, -0.0078125f, s);  // exact
-  return exp_grid_finish(t, tab[(int)nf]);
+  const float t = fmaf(m - kExpGridMagic, -0.0078125f, s);  // exact
+  return exp_grid_finish(t, tab[float_to_bits(m) & 1023u]);  // n is in m's low bits
 }
 
 // E[n], built at compile time in double-double arithmetic (error-free sums and products,

@@ -75,14 +75,10 @@ __device__ __forceinline__ float ex2_approx(float x) {
 __device__ __forceinline__ float fast_exp(float x) { return ex2_approx(__fmul_rn(x, kLog2e)); }
 
 // sigma = 0.5 (A dx dx + C dy dy) + B dx dy for a pair of pixels, operation for operation as
-// the reference (rasterize.rs:236), one rounding per operation (f2_mul is never contracted).
-// Also returns A dx, C dy and B dx for the gradients. A zero product may carry the other
-// sign than the scalar one; no decision on sigma depends on the sign of a zero.
-__device__ __forceinline__ f2 paired_sigma(f2 A, f2 B, f2 C, f2 dx, f2 dy, f2* adx, f2* cdy, f2* bdx) {
-  *adx = f2_mul(A, dx);
-  *cdy = f2_mul(C, dy);
-  *bdx = f2_mul(B, dx);
-  return f2_add(f2_mul(f2_splat(0.5f), f2_add(f2_mul(*adx, dx), f2_mul(*cdy, dy))), f2_mul(*bdx, dy));
+// the reference (rasterize.rs:236), one rounding per operation (f2_mul is never contracted);
+// cdyy = (C dy) dy.
+__device__ __forceinline__ f2 paired_sigma(f2 A, f2 B, f2 dx, f2 dy, f2 cdyy) {
+  return f2_add(f2_mul(f2_splat(0.5f), f2_add(f2_mul(f2_mul(A, dx), dx), cdyy)), f2_mul(f2_mul(B, dx), dy));
 }
 
 __device__ __forceinline__ bool evaluate_bwd(float px, float py, float mx, float my, float A, float B, float C,
@@ -156,10 +152,9 @@ __global__ void diag_pair_exact_kernel(uint32_t n, unsigned int* __restrict__ mi
     const float A = diag_uniform(i, 1u, 0.0f, 3.4f), B = diag_uniform(i, 2u, -1.7f, 1.7f);
     const float C = diag_uniform(i, 3u, 0.0f, 3.4f), dx = diag_uniform(i, 4u, -48.0f, 48.0f);
     const float dy0 = diag_uniform(i, 5u, -48.0f, 48.0f), dy1 = diag_uniform(i, 6u, -48.0f, 48.0f);
-    f2 adx, cdy, bdx;
+    const f2 dy2 = f2_make(dy0, dy1), cdyy = f2_mul(f2_mul(f2_splat(C), dy2), dy2);
     float p0, p1;
-    f2_split(paired_sigma(f2_splat(A), f2_splat(B), f2_splat(C), f2_splat(dx), f2_make(dy0, dy1), &adx, &cdy, &bdx),
-             p0, p1);
+    f2_split(paired_sigma(f2_splat(A), f2_splat(B), f2_splat(dx), dy2, cdyy), p0, p1);
     const float dys[2] = {dy0, dy1}, ps[2] = {p0, p1};
 #pragma unroll
     for (int q = 0; q < 2; q++) {
@@ -561,10 +556,7 @@ __global__ void __launch_bounds__(32 * FwdShape<TW, TH>::kWarps, 32 / FwdShape<T
           const float dx = px - e0.x, dy = py - e0.y;
           const float sigma = 0.5f * (e0.z * dx * dx + e1.x * dy * dy) + e0.w * dx * dy;
           const bool in = sigma >= 0.0f && sigma <= e1.z;
-          const float sg = in ? sigma : crm::kExpGridSkip;
-          const float mm = __fmaf_rn(sg, 128.0f, crm::kExpGridMagic);
-          const float t = __fmaf_rn(mm - crm::kExpGridMagic, -0.0078125f, sg);
-          const float og = e1.y * crm::exp_grid_finish(t, tab[fbits(mm) & 1023u]);
+          const float og = e1.y * crm::expf_cr_grid(in ? sigma : crm::kExpGridSkip, tab);
           float alpha = og < SPLAT_ALPHA_MIN ? 0.0f : fminf(og, SPLAT_ALPHA_MAX);
           float test_t = T * (1.0f - alpha);
           if (test_t < SPLAT_T_MIN) {  // the pixel is done without this entry
@@ -961,7 +953,7 @@ __device__ __forceinline__ void evaluate_row(BwdStage& st, uint32_t e, uint32_t 
   for (int c = 0; c < 8; c++) {
     const f2 dx = f2_sub(px, mx);
     px = f2_add(px, one);
-    const f2 sigma = f2_add(f2_mul(f2_splat(0.5f), f2_add(f2_mul(f2_mul(A, dx), dx), cdyy)), f2_mul(f2_mul(B, dx), dy));
+    const f2 sigma = paired_sigma(A, B, dx, dy, cdyy);
     float s0, s1, t0, t1;
     f2_split(sigma, s0, s1);
     f2_split(f2_sub(sigma, f2_splat(sure)), t0, t1);
