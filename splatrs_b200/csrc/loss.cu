@@ -400,29 +400,24 @@ __global__ void __launch_bounds__(kLossThreads) ssim_bwd_kernel(const float* __r
 constexpr int kRun = 4;
 constexpr int kTileW = kLossTile;
 constexpr int kEdgeW = kTileW + 2 * kHalo;
-template <int TH>
-struct SmallShape {
-  static constexpr int kEdgeH = TH + 2 * kHalo;
-  static constexpr int kItemsH = kEdgeH * (kTileW / kRun), kItemsV = kTileW * (TH / kRun);
-  static constexpr int kThreads = (kItemsH + 31) / 32 * 32;
-  static_assert(kItemsV <= kThreads, "a thread takes one run per pass");
-};
+constexpr int kTileH = 16, kEdgeH = kTileH + 2 * kHalo;
+constexpr int kItemsH = kEdgeH * (kTileW / kRun), kItemsV = kTileW * (kTileH / kRun);
+constexpr int kSmallThreads = (kItemsH + 31) / 32 * 32;
+static_assert(kItemsV <= kSmallThreads, "a thread takes one run per pass");
 // Row strides in shared memory: 8 rows of 16-byte accesses at one column hit distinct banks.
 constexpr int kStride2 = 42, kStride1 = 44, kStrideH2 = 34, kStrideH1 = 36;
-template <int TH>
 struct FwdTile {
-  float2 xy[SmallShape<TH>::kEdgeH][kStride2];                                       // (prediction, target)
-  float2 h01[SmallShape<TH>::kEdgeH][kStrideH2], h23[SmallShape<TH>::kEdgeH][kStrideH2];  // horizontal blurs of (x, y), (x^2, y^2)
-  float h4[SmallShape<TH>::kEdgeH][kStrideH1];                                       // and of x y
-  double red[3][SmallShape<TH>::kThreads / 32];
+  float2 xy[kEdgeH][kStride2];                            // (prediction, target)
+  float2 h01[kEdgeH][kStrideH2], h23[kEdgeH][kStrideH2];  // horizontal blurs of (x, y), (x^2, y^2)
+  float h4[kEdgeH][kStrideH1];                            // and of x y
+  double red[3][kSmallThreads / 32];
 };
-template <int TH>
 struct BwdTile {
-  float2 m01[SmallShape<TH>::kEdgeH][kStride2];  // partial maps w.r.t. mu_x and E[x^2]
-  float m2[SmallShape<TH>::kEdgeH][kStride1];    // and w.r.t. E[xy]
-  float2 h01[SmallShape<TH>::kEdgeH][kStrideH2];
-  float h2[SmallShape<TH>::kEdgeH][kStrideH1];
-  double red[3][SmallShape<TH>::kThreads / 32];
+  float2 m01[kEdgeH][kStride2];  // partial maps w.r.t. mu_x and E[x^2]
+  float m2[kEdgeH][kStride1];    // and w.r.t. E[xy]
+  float2 h01[kEdgeH][kStrideH2];
+  float h2[kEdgeH][kStrideH1];
+  double red[3][kSmallThreads / 32];
 };
 
 // One tap of an output's running sums: acc[o] += w_k v for the outputs o that input q reaches.
@@ -455,20 +450,18 @@ __device__ __forceinline__ void store_run(float* dst, const float a[kRun]) {
 
 // Per-pixel SSIM and its partial maps; the block's sums of SSIM, |x - y| and the squared
 // clamped error (PSNR) go to partial[3 * block].
-template <int TH>
-__global__ void __launch_bounds__(SmallShape<TH>::kThreads) ssim_fwd_small_kernel(
+__global__ void __launch_bounds__(kSmallThreads) ssim_fwd_small_kernel(
     const float* __restrict__ pred, const void* __restrict__ target_arg, int target_u8, uint32_t width_arg,
     uint32_t height_arg, LossKernel K, float* __restrict__ dmaps, double* __restrict__ partial,
     const StepParams* __restrict__ sp) {
   chain_begin();
-  typedef SmallShape<TH> S;
   extern __shared__ __align__(16) unsigned char loss_smem[];
-  FwdTile<TH>& t = *reinterpret_cast<FwdTile<TH>*>(loss_smem);
+  FwdTile& t = *reinterpret_cast<FwdTile*>(loss_smem);
   const void* target = sp ? sp->target : target_arg;
-  const int ox = blockIdx.x * kTileW, oy = blockIdx.y * TH;
+  const int ox = blockIdx.x * kTileW, oy = blockIdx.y * kTileH;
   const int width = (int)width_arg, height = (int)height_arg, ch = blockIdx.z, tid = threadIdx.x;
   const float c1 = 0.01f * 0.01f, c2 = 0.03f * 0.03f;
-  for (int i = tid; i < S::kEdgeH * kEdgeW; i += S::kThreads) {
+  for (int i = tid; i < kEdgeH * kEdgeW; i += kSmallThreads) {
     const int r = i / kEdgeW, c = i % kEdgeW;
     const int gy = oy - kHalo + r, gx = ox - kHalo + c;
     float vx = 0.0f, vy = 0.0f;
@@ -484,8 +477,8 @@ __global__ void __launch_bounds__(SmallShape<TH>::kThreads) ssim_fwd_small_kerne
   for (int k = 0; k < 6; k++) wp[k] = f2_splat(K.w[k]);
   __syncthreads();
   // Horizontal pass (loss.rs:42-56) of every row with its halo.
-  if (tid < S::kItemsH) {
-    const int r = tid % S::kEdgeH, c0 = tid / S::kEdgeH * kRun;
+  if (tid < kItemsH) {
+    const int r = tid % kEdgeH, c0 = tid / kEdgeH * kRun;
     f2 a01[kRun], a23[kRun];
     float a4[kRun];
 #pragma unroll
@@ -511,7 +504,7 @@ __global__ void __launch_bounds__(SmallShape<TH>::kThreads) ssim_fwd_small_kerne
   __syncthreads();
   // Vertical pass (loss.rs:58-70) and per-pixel SSIM (loss.rs:101-119).
   double s_ssim = 0.0, s_l1 = 0.0, s_se = 0.0;
-  if (tid < S::kItemsV) {
+  if (tid < kItemsV) {
     const int c = tid % kTileW, r0 = tid / kTileW * kRun;
     f2 m01[kRun], e23[kRun];
     float e4[kRun];
@@ -576,7 +569,7 @@ __global__ void __launch_bounds__(SmallShape<TH>::kThreads) ssim_fwd_small_kerne
   __syncthreads();
   if (tid < 3) {
     double v = 0.0;
-    for (int w = 0; w < S::kThreads / 32; w++) v += t.red[tid][w];
+    for (int w = 0; w < kSmallThreads / 32; w++) v += t.red[tid][w];
     const size_t block = ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 3 + ch;
     partial[3 * block + tid] = v;
   }
@@ -584,24 +577,22 @@ __global__ void __launch_bounds__(SmallShape<TH>::kThreads) ssim_fwd_small_kerne
 
 // Gradient of the loss w.r.t. the prediction (loss.rs:124-133, :155-169); the first block also
 // finishes the loss values.
-template <int TH>
-__global__ void __launch_bounds__(SmallShape<TH>::kThreads) ssim_bwd_small_kernel(
+__global__ void __launch_bounds__(kSmallThreads) ssim_bwd_small_kernel(
     const float* __restrict__ pred, const void* __restrict__ target_arg, int target_u8, uint32_t width_arg,
     uint32_t height_arg, LossKernel K, const float* __restrict__ dmaps, const double* __restrict__ partial,
     float lambda, float* __restrict__ grad, float* __restrict__ out3, const StepParams* __restrict__ sp) {
   chain_begin();
-  typedef SmallShape<TH> S;
   extern __shared__ __align__(16) unsigned char loss_smem[];
-  BwdTile<TH>& t = *reinterpret_cast<BwdTile<TH>*>(loss_smem);
+  BwdTile& t = *reinterpret_cast<BwdTile*>(loss_smem);
   if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) {
-    finalize_loss<S::kThreads>(partial, 3 * gridDim.x * gridDim.y, 3 * (uint64_t)width_arg * height_arg, lambda,
+    finalize_loss<kSmallThreads>(partial, 3 * gridDim.x * gridDim.y, 3 * (uint64_t)width_arg * height_arg, lambda,
                                t.red, out3);
   }
   const void* target = sp ? sp->target : target_arg;
-  const int ox = blockIdx.x * kTileW, oy = blockIdx.y * TH;
+  const int ox = blockIdx.x * kTileW, oy = blockIdx.y * kTileH;
   const int width = (int)width_arg, height = (int)height_arg, ch = blockIdx.z, tid = threadIdx.x;
   const size_t npix = (size_t)width * height;
-  for (int i = tid; i < S::kEdgeH * kEdgeW; i += S::kThreads) {
+  for (int i = tid; i < kEdgeH * kEdgeW; i += kSmallThreads) {
     const int r = i / kEdgeW, c = i % kEdgeW;
     const int gy = oy - kHalo + r, gx = ox - kHalo + c;
     float m0 = 0.0f, m1 = 0.0f, m2 = 0.0f;
@@ -619,8 +610,8 @@ __global__ void __launch_bounds__(SmallShape<TH>::kThreads) ssim_bwd_small_kerne
   for (int k = 0; k < 6; k++) wp[k] = f2_splat(K.w[k]);
   __syncthreads();
   // The blur of the three partial maps (the blur is self-adjoint, loss.rs:124-127).
-  if (tid < S::kItemsH) {
-    const int r = tid % S::kEdgeH, c0 = tid / S::kEdgeH * kRun;
+  if (tid < kItemsH) {
+    const int r = tid % kEdgeH, c0 = tid / kEdgeH * kRun;
     f2 a01[kRun];
     float a2[kRun];
 #pragma unroll
@@ -641,7 +632,7 @@ __global__ void __launch_bounds__(SmallShape<TH>::kThreads) ssim_bwd_small_kerne
     store_run(&t.h2[r][c0], a2);
   }
   __syncthreads();
-  if (tid < S::kItemsV) {
+  if (tid < kItemsV) {
     const int c = tid % kTileW, r0 = tid / kTileW * kRun;
     f2 b01[kRun];
     float b2[kRun];
@@ -692,8 +683,6 @@ LossKernel make_loss_kernel() {
   return k;
 }
 
-constexpr int kSmallTileH = 16;
-
 Status launch_loss(Ctx* c, const float* pred, const void* target, int target_u8, uint32_t width, uint32_t height,
                    float lambda, float* grad, float* out3, const StepParams* sp, const BatchTable* bt,
                    uint32_t blocks_cap, uint64_t pix_cap) {
@@ -703,7 +692,7 @@ Status launch_loss(Ctx* c, const float* pred, const void* target, int target_u8,
   const uint64_t tiles = (uint64_t)ceil_div(width, kLT) * ceil_div(height, kLT);
   const bool small = !bt && tiles < 4 * (uint64_t)c->sm_count;
   const dim3 grid = bt      ? dim3(blocks_cap)
-                    : small ? dim3(ceil_div(width, kTileW), ceil_div(height, kSmallTileH), 3)
+                    : small ? dim3(ceil_div(width, kTileW), ceil_div(height, kTileH), 3)
                             : dim3(ceil_div(width, kLT), ceil_div(height, kLT));
   float* dmaps = nullptr;
   double* sums = nullptr;
@@ -711,14 +700,11 @@ Status launch_loss(Ctx* c, const float* pred, const void* target, int target_u8,
   SPLAT_TRY(arena_reserve(c, (size_t)grid.x * grid.y * grid.z * 3 * 8, (void**)&sums));
   const LossKernel K = make_loss_kernel();
   if (small) {
-    typedef SmallShape<kSmallTileH> S;
-    static_assert(sizeof(FwdTile<kSmallTileH>) <= 48 * 1024 && sizeof(BwdTile<kSmallTileH>) <= 48 * 1024, "");
-    SPLAT_TRY(launch_chained(c, "ssim_fwd_small_kernel", ssim_fwd_small_kernel<kSmallTileH>, grid, S::kThreads,
-                             sizeof(FwdTile<kSmallTileH>), pred, target, target_u8, width, height, K, dmaps, sums,
-                             sp));
-    SPLAT_TRY(launch_chained(c, "ssim_bwd_small_kernel", ssim_bwd_small_kernel<kSmallTileH>, grid, S::kThreads,
-                             sizeof(BwdTile<kSmallTileH>), pred, target, target_u8, width, height, K, dmaps, sums,
-                             lambda, grad, out3, sp));
+    static_assert(sizeof(FwdTile) <= 48 * 1024 && sizeof(BwdTile) <= 48 * 1024, "");
+    SPLAT_TRY(launch_chained(c, "ssim_fwd_small_kernel", ssim_fwd_small_kernel, grid, kSmallThreads, sizeof(FwdTile),
+                             pred, target, target_u8, width, height, K, dmaps, sums, sp));
+    SPLAT_TRY(launch_chained(c, "ssim_bwd_small_kernel", ssim_bwd_small_kernel, grid, kSmallThreads, sizeof(BwdTile),
+                             pred, target, target_u8, width, height, K, dmaps, sums, lambda, grad, out3, sp));
   } else {
     SPLAT_TRY(launch_chained(c, "ssim_fwd_kernel", ssim_fwd_kernel, grid, kLossThreads, 0, pred, target, target_u8,
                              width, height, K, dmaps, sums, sp, bt));
