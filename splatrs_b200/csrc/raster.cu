@@ -1,16 +1,16 @@
 // Front-to-back alpha compositing, forward and backward (reference src/rasterize.rs).
 //
-// The forward and the default backward give every warp an 8x8 pixel sub-block of a tile (two
-// pixels per lane, computed as f32x2 pairs) and let it walk the tile's sorted list by itself:
-// it scans 64 entries at a time for those whose pixel rectangle touches its sub-block, stages
-// their records 32 at a time in its own shared memory (gathered while the previous 32 are
-// composited) and never meets the block's other warps at a barrier. The one-pixel-per-thread
-// backward and the deterministic one run one block per tile instead and stage chunks for the
-// whole block. Tile shape (16x16 by default; 8x8 and 16x32 too) and, for the one-pixel
-// backward, chunk depth are template parameters chosen at run time from the context's
-// configuration (the autotuner's pick). Every per-pixel decision (sigma range, alpha >= 1/255,
-// the 0.99 clamp, T < 1e-4) is taken on values computed exactly as the reference computes
-// them: unfused arithmetic and a correctly rounded exp.
+// The forward gives every warp an 8x4 pixel sub-block of a tile, one pixel per lane in scalar
+// arithmetic; the default backward an 8x8 one, two pixels per lane as f32x2 pairs. The tile's
+// warps scan its sorted list together, 1,024 entries at a time with barriers around each scan,
+// for the sub-blocks that an entry's pixel rectangle touches; every warp then walks the entries
+// of its own sub-block alone, staging records in its own shared memory (32 at a time, 16 in the
+// backward, gathered while the ones before are composited). The one-pixel-per-thread backward
+// and the deterministic one stage chunks for the whole block. Tile shape (16x16 by default; 8x8
+// and 16x32 too) and, for the one-pixel backward, chunk depth are template parameters chosen at
+// run time from the context's configuration (the autotuner's pick). Every per-pixel decision
+// (sigma range, alpha >= 1/255, the 0.99 clamp, T < 1e-4) is taken on values computed exactly as
+// the reference computes them: unfused arithmetic and a correctly rounded exp.
 #include <mutex>
 #include <set>
 #include <type_traits>
@@ -1617,14 +1617,16 @@ Status launch_raster_bwd(Ctx* c, const float* proj, const uint32_t* gauss, const
       c, raster_bwd_x2_kernel<TW, TH, K, R>, blocks, reinterpret_cast<const float4*>(proj), gauss,                  \
       reinterpret_cast<const uint2*>(ranges), blocks, width, height, tiles_x, bg[0], bg[1], bg[2], final_t,      \
       n_contrib, dimage, reinterpret_cast<float4*>(pgrad), cap, reinterpret_cast<unsigned long long*>(pairs), bt)))
-// A view whose warps fit the GPU at 16 warps per SM takes the build with 122 registers and no
-// spills, a larger one 20 warps per SM in 96 registers (measured before phase 2 was branch-free:
-// 34k Gaussians at 256x256 88 us against 97, 2k at 128x96 29 against 31; 1M at 1920x1080 689 against
-// 677, 100k at 1280x720 68 against 66).
-#define SPLAT_BWD2(TW, TH)                                                                                  \
-  const bool resident = (uint64_t)blocks * BwdShape<TW, TH>::W::kPerTile <= (uint64_t)c->sm_count * 16;    \
-  if (pairs) SPLAT_BWD2X(TW, TH, true, 16); else if (resident) SPLAT_BWD2X(TW, TH, false, 16);            \
-  else SPLAT_BWD2X(TW, TH, false, 20)
+// 16 warps per SM in up to 128 registers, or, for views of many 16x16 tiles, 20 warps in 96. The
+// line lies at 16 tiles per SM (2,368): 16 against 20 warps 22.9 / 24.0 us at 128x96 (2k Gaussians),
+// 78.8 / 83.5 at 256x256 (34k), 84.4 / 90.2 at 640x480 (34k, 1,200 tiles), 53.5 / 54.4 at 800x600
+// (100k, 1,900 tiles); 65.1 / 62.5 at 1280x720 (100k, 3,600 tiles), 256 / 256 at 1297x840 (187k),
+// 674 / 666 at 1920x1080 (1M). 8x8 tiles spill at 20 warps and are 8-25% slower at every size
+// (668 / 737 us in the last); a 16x32 block has eight warps, so two blocks per SM either way.
+#define SPLAT_BWD2(TW, TH)                                                                                   \
+  constexpr int kMany = TW == 16 && TH == 16 ? 20 : 16;                                                      \
+  if (pairs) SPLAT_BWD2X(TW, TH, true, 16); else if (blocks <= 16u * (uint32_t)c->sm_count)                  \
+    SPLAT_BWD2X(TW, TH, false, 16); else SPLAT_BWD2X(TW, TH, false, kMany)
   if (rc.ppl == 2) {
     if (rc.tile_w == 16 && rc.tile_h == 16) {
       SPLAT_BWD2(16, 16);
