@@ -195,12 +195,14 @@ RASTER_BWD_BYTES_PER_PIXEL = 20    # dL/dpix (12) + final T (4) + n_contrib (4) 
 RASTER_BYTES_PER_ENTRY = 52        # sorted index (4) + record gather (48)
 # dram__bytes_read.sum + dram__bytes_write.sum per launch, ncu, default workload.
 # By kernel, tile and the backward's pixels per thread: the chunk depth moves the figures by 1%.
-NCU_DRAM_BYTES_1M = {("raster_bwd", 16, 16, 1): int((197.05 + 17.84) * 1e6),
-                     ("raster_fwd", 16, 16, 1): int((82.84 + 20.76) * 1e6),
-                     ("raster_bwd", 16, 16, 2): int((198.23 + 20.35) * 1e6),
-                     ("raster_fwd", 16, 16, 2): int((83.22 + 21.74) * 1e6),
-                     ("raster_bwd", 16, 32, 2): int((185.54 + 13.20) * 1e6),
-                     ("raster_fwd", 16, 32, 2): int((74.59 + 16.79) * 1e6)}
+NCU_DRAM_BYTES_1M = {("raster_bwd", 16, 16, 1): int((197.60 + 17.64) * 1e6),
+                     ("raster_fwd", 16, 16, 1): int((83.17 + 21.00) * 1e6),
+                     ("raster_bwd", 16, 16, 2): int((198.37 + 19.71) * 1e6),
+                     ("raster_fwd", 16, 16, 2): int((83.18 + 21.89) * 1e6),
+                     ("raster_bwd", 16, 32, 2): int((187.04 + 15.40) * 1e6),
+                     ("raster_fwd", 16, 32, 2): int((75.93 + 18.75) * 1e6),
+                     ("raster_bwd", 8, 8, 2): int((202.22 + 19.03) * 1e6),
+                     ("raster_fwd", 8, 8, 2): int((88.53 + 22.19) * 1e6)}
 RASTER_FWD_FLOP_PER_PAIR = 20
 RASTER_BWD_FLOP_PER_PAIR = 50
 RASTER_FWD_SFU_PER_PAIR = 1        # one exp

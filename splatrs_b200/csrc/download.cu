@@ -2,7 +2,7 @@
 // pinned nor, often, mapped yet. The device converts and copies 44 MB in a millisecond; the rest of
 // the 10 ms that a fresh array took was its pages' first touch, taken one by one under the driver's
 // single-threaded copy. Here several threads touch them, while the device converts the records:
-// 187k Gaussians 15.4 -> 8-12 ms, or 9.8 -> 8.1 on another machine, and no slower the first time.
+// 187k Gaussians 9.8-15.4 -> 6.7-11.7 ms by machine, and no slower the first time.
 // (Pinned slots emptied by several threads were faster on a repeated call, 4.3 ms, but their
 // allocation made a context's first call 3-20 ms longer.)
 #include <algorithm>

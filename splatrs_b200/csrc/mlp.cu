@@ -717,7 +717,7 @@ __global__ void __launch_bounds__(kTcRows) mlp_forward_tc_kernel(const float* __
 // lanes of each warp and kept in registers. Rounding points are those of the mma.sync kernel
 // and the oracle's bf16 mode.
 //
-// A tile is seven dependent steps of MMA, wait and epilogue: latency, not a rate, bounds it,
+// A tile is six dependent steps of MMA, wait and epilogue: latency, not a rate, bounds it,
 // so the point is to have two CTAs on an SM. That takes half of the tensor memory (224
 // columns of 512: z1 is multiplied out again, beside dh1, instead of being kept, and z3
 // shares its columns with dh2 and dh1) and no staging tile for the bias gradients. 65,536

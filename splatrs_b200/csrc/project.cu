@@ -858,9 +858,9 @@ __device__ __forceinline__ void adam_planes(AdamStage<NT, kAhead>& st, const Ada
 // and v, over every plane (zero gradients still decay the moments, adam.rs:56-60).
 // Four blocks of 128 per SM: the 59 gradients and the streamed parameters and moments
 // would take 190-242 registers (8 warps per SM, too few to hide the memory latency of an
-// HBM-bound kernel); capped at 128 the kernel spills a few hundred bytes to L1 and runs
-// 22-23% faster (measured at 1M Gaussians: 0.606 -> 0.475 ms with Adam, 0.149 -> 0.115 ms
-// without).
+// HBM-bound kernel); capped at 128 the kernel spills some hundred bytes to L1 at SH degrees 2 and
+// 3 and ran 22-23% faster (with the optimiser's operands still in registers: 0.606 -> 0.475 ms
+// with Adam at 1M Gaussians, 0.149 -> 0.115 without; now 0.33 and 0.13 ms).
 constexpr int kAdamAhead = 3;  // 5 and 7 were no faster; 3 leaves room for the gradient columns in 48 KB
 template <int DEG, bool ADAM, bool BF16>
 __global__ void __launch_bounds__(128, 4) project_bwd_kernel(const float4* __restrict__ planes, int64_t n, int64_t cap,

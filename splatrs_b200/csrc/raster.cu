@@ -900,8 +900,8 @@ constexpr float kSigmaEdge = 1e-4f;
 // The phases hand (gauss) and (h, w) over in two 8 x 32 arrays of pairs in shared memory.
 // Against one pixel pair per lane for everything (records broadcast from shared memory with
 // each scalar duplicated, a 13-shuffle reduction of 12 slots over the warp for every entry)
-// this takes about 130 instead of 185 warp instructions per entry. Bound by latency and issue
-// (63% of the issue slots, FMA pipe 48%, shared-memory reads 60%; DRAM 3% of its peak).
+// this takes about 134 instead of 185 warp instructions per entry. Bound by latency and issue
+// (62% of the issue slots, FMA pipe 52%, shared-memory accesses 56%; DRAM 5% of its peak).
 // Time: 1M Gaussians at 1920x1080 975 -> 666 us, 187k clustered at 1297x840 377 -> 257, 34k at
 // 256x256 164 -> 79, 20k wide ones at 1386x1080 163 -> 117. kCount adds the evaluated-pair
 // counter (untimed diagnostics only).
